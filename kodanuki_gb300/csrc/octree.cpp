@@ -556,6 +556,16 @@ struct Node {
 	double radius = 0.0;
 	bool negation = false; // fma(x, -1, 0): -x
 	bool product  = false; // fma(x, y, 0) from a multiplication
+	// a fused step (world.h MarchForm): its parameters as they are written,
+	// how far an axis has come (the terms taken so far), and the single steps
+	// it stands for
+	uint8_t form  = FormFma, flags = 0;
+	Operand m;             // FormNorm: the inside term
+	float params[4] = { 0.0f, 0.0f, -0.0f, 0.0f };
+	uint8_t stage = 0;     // FormAxis: 0 none, 1 c, 2 a side, 3 h, 4 r, 5 e; else 1 once e is taken
+	uint32_t took = 1;
+	Operand single;        // FormAxis of one step: that step's a and post
+	uint8_t singlePost = PostNone;
 };
 
 // sdf/program.cpp:57 runStep in double, for steps of constants alone.
@@ -621,6 +631,338 @@ struct Lowering {
 		Operand r = make(n, from);
 		r.shared  = true;
 		return r;
+	}
+};
+
+// The steps the result needs, and how often each is read.
+struct Readers {
+	std::vector<uint8_t> live;
+	std::vector<uint32_t> uses;
+};
+bool readsW(const Node& n) { return n.post == PostMin || n.post == PostMax || n.post == PostSminK; }
+template <typename F>
+void eachOperand(const Node& n, const F& read) {
+	if (n.form == FormSphere) {
+		if (readsW(n)) read(n.w);
+		return;
+	}
+	read(n.a);
+	if (n.form != FormAxis) {
+		read(n.b);
+		read(n.c);
+	}
+	if (readsW(n)) read(n.w);
+	if (n.form == FormNorm) read(n.m);
+}
+Readers readersOf(const std::vector<Node>& nodes, uint32_t result) {
+	Readers r;
+	r.live.assign(nodes.size(), 0);
+	r.uses.assign(nodes.size(), 0);
+	r.live[result] = 1;
+	r.uses[result] = 1;
+	for (size_t j = nodes.size(); j-- > 0;) {
+		if (!r.live[j]) continue;
+		eachOperand(nodes[j], [&](const Operand& o) {
+			if (o.kind != Operand::Node) return;
+			r.live[o.node] = 1;
+			r.uses[o.node] += 1;
+		});
+	}
+	return r;
+}
+
+// Fuse the runs of single steps that signed distances are made of (world.h
+// MarchForm).  Each rule takes single steps that nothing else reads into the
+// step that reads them, and keeps every rounding they make: a term left out
+// is an exact zero, sums are only turned about (x + y = y + x), and a maximum
+// or minimum keeps which operand it compares with which.
+struct Fusing {
+	std::vector<Node>& nodes;
+	Readers reads;
+
+	static bool is(const Operand& o, uint8_t slot) { return o.kind == Operand::Reserved && o.slot == slot; }
+	static bool point(const Operand& o) { return o.kind == Operand::Reserved && o.slot >= SlotX && o.slot <= SlotZ; }
+	static bool same(const Operand& a, const Operand& b) {
+		if (a.kind != b.kind || a.kind == Operand::Immediate) return false;
+		return a.kind == Operand::Node ? a.node == b.node : a.slot == b.slot;
+	}
+	// the step an operand reads, where this is its only reader
+	Node* only(const Operand& o, uint32_t readers = 1) const {
+		return o.kind == Operand::Node && reads.uses[o.node] == readers && !nodes[o.node].rare ? &nodes[o.node] : nullptr;
+	}
+	// x - value, as fma(value, -1, x); x + value or value + x, as fma(., 1, .);
+	// value - x, as fma(x, -1, value)
+	enum Sum { NoSum, Minus, Plus, From };
+	static Sum sumWith(const Node& n, Operand& x, double& value) {
+		if (n.rare || n.form != FormFma) return NoSum;
+		if (n.a.kind == Operand::Immediate && is(n.b, SlotMinusOne) && n.c.kind != Operand::Immediate) {
+			x     = n.c;
+			value = n.a.value;
+			return Minus;
+		}
+		if (is(n.b, SlotOne) && (n.a.kind == Operand::Immediate) != (n.c.kind == Operand::Immediate)) {
+			x     = n.a.kind == Operand::Immediate ? n.c : n.a;
+			value = n.a.kind == Operand::Immediate ? n.a.value : n.c.value;
+			return Plus;
+		}
+		if (is(n.b, SlotMinusOne) && n.c.kind == Operand::Immediate && n.a.kind != Operand::Immediate) {
+			x     = n.a;
+			value = n.c.value;
+			return From;
+		}
+		return NoSum;
+	}
+	// x itself, as fma(x, 1, 0)
+	static bool copyOf(const Node& n, Operand& x) {
+		if (n.rare || n.form != FormFma || !is(n.b, SlotOne) || !is(n.c, SlotZero) || n.a.kind == Operand::Immediate) return false;
+		x = n.a;
+		return true;
+	}
+
+	// max(q, 0) + min(q, 0) = q, which max and min made of one step
+	void joined(Node& n) {
+		if (n.rare || n.form != FormFma || !is(n.b, SlotOne)) return;
+		const Node* s[2] = { only(n.a), only(n.c) };
+		if (!s[0] || !s[1]) return;
+		Operand q[2];
+		for (int k = 0; k < 2; ++k) {
+			if (!copyOf(*s[k], q[k]) || !readsW(*s[k]) || s[k]->w.kind != Operand::Immediate || s[k]->w.value != 0.0) return;
+		}
+		if (!((s[0]->post == PostMax && s[1]->post == PostMin) || (s[0]->post == PostMin && s[1]->post == PostMax)) || !same(q[0], q[1])) return;
+		const uint32_t took = n.took + s[0]->took + s[1]->took;
+		if (const Node* whole = only(q[0], 2); whole && n.post == PostNone) {
+			n = *whole;
+			n.took += took;
+		} else {
+			n.a    = q[0];
+			n.c    = Operand();
+			n.took = took;
+		}
+	}
+
+	// a coordinate's distance to a slab, a term at a time
+	void axis(Node& n) {
+		Operand x;
+		double value = 0.0;
+		const Sum sum = sumWith(n, x, value);
+		Node f        = n;
+		f.form        = FormAxis;
+		f.single      = n.a;
+		f.singlePost  = n.post;
+		if (sum != NoSum && point(x)) {
+			f.a         = x;
+			f.params[0] = sum == Plus ? -float(value) : float(value);
+			f.flags     = sum == From ? SideNegative : SideNone;
+			f.stage     = sum == From ? 2 : 1;
+			if (n.post == PostAbs && sum != From) {
+				f.post  = PostNone;
+				f.flags = SideAbs;
+				f.stage = 2;
+			}
+			n = f;
+			return;
+		}
+		const bool copied  = sum == NoSum && copyOf(n, x);
+		const bool negated = sum == NoSum && !copied && !n.rare && n.form == FormFma && is(n.b, SlotMinusOne) && is(n.c, SlotZero) && n.a.kind != Operand::Immediate;
+		if (negated) x = n.a;
+		if (copied && point(x)) { // the coordinate itself
+			f.a     = x;
+			f.stage = 1;
+			if (n.post == PostAbs) {
+				f.post  = PostNone;
+				f.flags = SideAbs;
+				f.stage = 2;
+			}
+			n = f;
+			return;
+		}
+		const Node* before = only(x);
+		if (!before || before->form != FormAxis || before->post != PostNone) return;
+		const uint8_t stage = before->stage;
+		for (int k = 0; k < 4; ++k) f.params[k] = before->params[k];
+		f.a     = before->a;
+		f.flags = before->flags;
+		f.took  = before->took + n.took;
+		if (negated || copied) {
+			if (stage != 1 || (copied && n.post != PostAbs)) return;
+			f.flags = negated ? SideNegative : SideAbs;
+			f.stage = 2;
+			if (copied) f.post = PostNone;
+		} else if (sum == Minus && stage <= 2) {
+			f.params[1] = float(value);
+			f.stage     = 3;
+		} else if (sum == Plus && stage <= 3) {
+			f.params[2] = float(value);
+			f.stage     = 4;
+		} else if (sum == Minus && stage <= 4) {
+			f.params[3] = float(value);
+			f.stage     = 5;
+		} else {
+			return;
+		}
+		n = f;
+	}
+
+	// the terms of a sum of squares, the first read last: each a slot, squared
+	// whole or its positive part, added by itself or by a fused multiply-add
+	struct Term {
+		Operand x;
+		bool positive = false, fused = false;
+		Node* strip   = nullptr; // a step that loses its square
+		uint32_t took = 0;
+	};
+	bool term(const Operand& o, Term& t) const {
+		Node* n = only(o);
+		if (!n) return false;
+		if (n->post == PostPosSq) {
+			t.positive = true;
+			if (!copyOf(*n, t.x)) {
+				t.x     = o;
+				t.strip = n;
+			} else {
+				t.took = n->took;
+			}
+			return true;
+		}
+		if (n->post == PostNone && n->form == FormFma && same(n->a, n->b) && n->a.kind == Operand::Node && is(n->c, SlotZero)) {
+			t.x    = n->a;
+			t.took = n->took;
+			return true;
+		}
+		return false;
+	}
+	bool terms(const Node& n, std::vector<Term>& out) const {
+		if (n.rare || n.form != FormFma || out.size() > 2) return false;
+		Operand rest;
+		Term t;
+		if (same(n.a, n.b) && n.a.kind == Operand::Node) { // fma(x, x, rest)
+			t.x     = n.a;
+			t.fused = true;
+			rest    = n.c;
+			out.push_back(t);
+		} else if (is(n.b, SlotOne)) { // a term and the rest
+			Term u, v;
+			const bool first = term(n.a, u), second = term(n.c, v);
+			if (first && second) { // the sum's first two
+				out.push_back(v);
+				out.push_back(u);
+				return true;
+			}
+			if (!first && !second) return false;
+			out.push_back(first ? u : v);
+			rest = first ? n.c : n.a;
+		} else {
+			return false;
+		}
+		Term last;
+		if (term(rest, last)) {
+			out.push_back(last);
+			return true;
+		}
+		const Node* s = only(rest);
+		if (!s || s->post != PostNone || out.size() > 2) return false;
+		const size_t at = out.size();
+		if (!terms(*s, out)) return false;
+		out[at].took += s->took;
+		return true;
+	}
+	void norm(Node& n) {
+		std::vector<Term> t;
+		if (n.post != PostSqrt || !terms(n, t) || t.size() < 2 || t.size() > 3) return;
+		std::reverse(t.begin(), t.end());
+		Node f  = n;
+		f.form  = FormNorm;
+		f.post  = PostNone;
+		f.flags = uint8_t(t.size() == 3 ? NormThree : 0);
+		f.c     = Operand();
+		Operand* slots[3] = { &f.a, &f.b, &f.c };
+		for (size_t k = 0; k < t.size(); ++k) {
+			if (t[k].x.kind == Operand::Immediate) return;
+			*slots[k] = t[k].x;
+			if (t[k].positive) f.flags |= uint8_t(NormPositive0 << k);
+			if (t[k].fused) f.flags |= uint8_t(k == 1 ? NormFused1 : NormFused2);
+			f.took += t[k].took;
+		}
+		for (const Term& k : t) {
+			if (k.strip) k.strip->post = k.strip->singlePost = PostNone;
+		}
+		f.params[0] = 0.0f;
+		f.stage     = 0;
+		// a point's distance to a centre: y first, then x and z by fused multiply-adds
+		const uint8_t order[3] = { SlotY, SlotX, SlotZ };
+		bool sphere            = f.flags == (NormThree | NormFused1 | NormFused2);
+		const Node* part[3]    = {};
+		for (int k = 0; k < 3 && sphere; ++k) {
+			part[k] = only(*slots[k], 2);
+			sphere  = part[k] && part[k]->form == FormAxis && part[k]->stage == 1 && part[k]->post == PostNone && is(part[k]->a, order[k]);
+		}
+		if (sphere) {
+			f.form  = FormSphere;
+			f.flags = 0;
+			f.params[0] = part[1]->params[0];
+			f.params[1] = part[0]->params[0];
+			f.params[2] = part[2]->params[0];
+			f.params[3] = 0.0f;
+			for (const Node* k : part) f.took += k->took;
+		}
+		n = f;
+	}
+	// the inside term of a box, and the rounding or the radius
+	void around(Node& n) {
+		Operand x;
+		double value = 0.0;
+		if (sumWith(n, x, value) == Minus) {
+			const Node* b = only(x);
+			if (!b || (b->form != FormNorm && b->form != FormSphere) || b->post != PostNone || b->stage != 0) return;
+			Node f  = *b;
+			f.post  = n.post;
+			f.w     = n.w;
+			f.radius = n.radius;
+			f.stage = 1;
+			f.took += n.took;
+			f.params[b->form == FormNorm ? 0 : 3] = float(value);
+			n = f;
+			return;
+		}
+		if (n.rare || n.form != FormFma || !is(n.b, SlotOne)) return;
+		for (int k = 0; k < 2; ++k) {
+			const Node* b = only(k == 0 ? n.a : n.c);
+			const Node* m = only(k == 0 ? n.c : n.a);
+			if (!b || !m || b->form != FormNorm || b->post != PostNone || b->stage != 0 || (b->flags & NormInside)) continue;
+			Operand h;
+			if (m->post != PostMin || m->w.kind != Operand::Immediate || m->w.value != 0.0 || !copyOf(*m, h)) continue;
+			Node f = *b;
+			f.post = n.post;
+			f.w    = n.w;
+			f.radius = n.radius;
+			f.flags |= NormInside;
+			f.m = h;
+			f.took += n.took + m->took;
+			// the inside term the terms' own maximum: max(a, max(b, c)), or max(a, b)
+			Operand p, q;
+			const Node* outer = only(h);
+			if (outer && outer->post == PostMax && copyOf(*outer, p) && same(p, f.a)) {
+				if (!(f.flags & NormThree) && same(outer->w, f.b)) {
+					f.flags |= NormInsideMax;
+					f.took += outer->took;
+				} else if (const Node* inner = only(outer->w); inner && (f.flags & NormThree) && inner->post == PostMax && copyOf(*inner, q) && same(q, f.b) && same(inner->w, f.c)) {
+					f.flags |= NormInsideMax;
+					f.took += outer->took + inner->took;
+				}
+				if (f.flags & NormInsideMax) f.m = Operand();
+			}
+			n = f;
+			return;
+		}
+	}
+	void run() {
+		for (size_t j = 0; j < nodes.size(); ++j) {
+			if (!reads.live[j] || nodes[j].rare) continue;
+			joined(nodes[j]);
+			axis(nodes[j]);
+			norm(nodes[j]);
+			around(nodes[j]);
+		}
 	}
 };
 
@@ -808,26 +1150,19 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 	// the result as a step
 	Operand result = val[p.result];
 	if (result.kind != Operand::Node) result = L.make(fma3(result, one, zero), p.result);
+	// what the counters count, then the fused form of it
+	const Readers single = readersOf(L.nodes, result.node);
+	out.marchSteps       = uint16_t(std::count(single.live.begin(), single.live.end(), 1));
+	Fusing { L.nodes, single }.run();
 	// the steps the result needs, and each one's last reader
-	const uint32_t m = uint32_t(L.nodes.size());
-	std::vector<uint8_t> live(m, 0);
-	live[result.node] = 1;
-	for (uint32_t j = m; j-- > 0;) {
-		if (!live[j]) continue;
-		const Node& x = L.nodes[j];
-		for (const Operand* o : { &x.a, &x.b, &x.c, &x.w }) {
-			if (o->kind == Operand::Node) live[o->node] = 1;
-		}
-	}
+	const uint32_t m                = uint32_t(L.nodes.size());
+	const std::vector<uint8_t> live = readersOf(L.nodes, result.node).live;
 	std::vector<uint32_t> lastRead(m, 0);
 	for (uint32_t j = 0; j < m; ++j) {
 		if (!live[j]) continue;
-		const Node& x   = L.nodes[j];
-		const bool usesW = x.post == PostMin || x.post == PostMax || x.post == PostSminK;
-		for (const Operand* o : { &x.a, &x.b, &x.c, &x.w }) {
-			if (o == &x.w && !usesW) continue;
-			if (o->kind == Operand::Node) lastRead[o->node] = std::max(lastRead[o->node], j);
-		}
+		eachOperand(L.nodes[j], [&](const Operand& o) {
+			if (o.kind == Operand::Node) lastRead[o.node] = std::max(lastRead[o.node], j);
+		});
 	}
 	lastRead[result.node] = m;
 	std::vector<uint8_t> slot(m, 0);
@@ -837,10 +1172,17 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 	out.march     = uint32_t(steps.size());
 	for (uint32_t j = 0; j < m; ++j) {
 		if (!live[j]) continue;
-		const Node& x    = L.nodes[j];
-		const bool usesW = x.post == PostMin || x.post == PostMax || x.post == PostSminK;
+		Node& x = L.nodes[j];
+		// an axis of one term costs no less fused than single, but where it is the whole program
+		if (x.form == FormAxis && x.took == 1 && j != result.node) {
+			x.form = FormFma;
+			x.a    = x.single;
+			x.post = x.singlePost;
+		}
+		const bool fused = x.form != FormFma;
+		const bool usesW = readsW(x);
 		MarchStep g      = {};
-		g.op             = x.rare ? uint8_t(kMarchRare + x.refOp) : x.post;
+		g.op             = x.rare ? uint8_t(kMarchRare + x.refOp) : uint8_t(x.form + x.post);
 		double immValue  = 0.0;
 		const auto slotOf = [&](const Operand& o) -> uint8_t {
 			if (o.kind == Operand::Node) return slot[o.node];
@@ -850,22 +1192,23 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 			}
 			return o.slot;
 		};
-		g.a       = slotOf(x.a);
-		g.b       = slotOf(x.b);
-		g.c       = slotOf(x.c);
+		if (x.form != FormSphere) g.a = slotOf(x.a);
+		if (x.form == FormFma || x.form == FormNorm) {
+			g.b = slotOf(x.b);
+			g.c = slotOf(x.c);
+		}
+		if (x.form == FormNorm) g.m = slotOf(x.m);
+		if (fused) g.flags = x.flags;
 		g.w       = usesW ? slotOf(x.w) : uint8_t(SlotZero);
 		g.value   = float(x.post == PostSminK ? x.radius : immValue);
 		g.quarter = x.post == PostSminK ? float(0.25 / x.radius) : 0.0f;
 		// free the slots read here for the last time (each value once)
-		const Operand* reads[4] = { &x.a, &x.b, &x.c, &x.w };
-		for (int r = 0; r < 4; ++r) {
-			const Operand* o = reads[r];
-			if (r == 3 && !usesW) continue;
-			if (o->kind != Operand::Node || lastRead[o->node] != j) continue;
-			bool first = true;
-			for (int q = 0; q < r; ++q) first = first && !(reads[q]->kind == Operand::Node && reads[q]->node == o->node);
-			if (first) freeSlots.push_back(slot[o->node]);
-		}
+		std::vector<uint32_t> freed;
+		eachOperand(x, [&](const Operand& o) {
+			if (o.kind != Operand::Node || lastRead[o.node] != j || std::count(freed.begin(), freed.end(), o.node)) return;
+			freed.push_back(o.node);
+			freeSlots.push_back(slot[o.node]);
+		});
 		if (!freeSlots.empty()) {
 			slot[j] = freeSlots.back();
 			freeSlots.pop_back();
@@ -877,6 +1220,14 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 		g.dst = slot[j];
 		steps.push_back(g);
 		++kept;
+		if (fused) {
+			MarchParams q;
+			std::copy(x.params, x.params + 4, q.v);
+			MarchStep unit;
+			std::memcpy(&unit, &q, sizeof unit);
+			steps.push_back(unit);
+			++kept;
+		}
 	}
 	out.marchCount = uint16_t(kept);
 	out.marchSlot  = slot[result.node];

@@ -109,40 +109,124 @@ KDN_HD void setPoint(float* slots, uint32_t stride, const float p[3]) {
 	slots[SlotZ * stride] = p[2];
 }
 
-// One step of the march form (world.h MarchStep): r = post(fma(a, b, c), w)
-// with the post operations worked out together and the step's picked, so
-// the lanes of a warp on different steps do not split; a rare step runs the
-// reference operation.  Writes the result to its slot and returns it.
-KDN_HD float marchStep(const MarchStep& s, float* slots, uint32_t stride) {
-	slots[SlotImm * stride] = s.value;
-	const float a = slots[s.a * stride], b = slots[s.b * stride], c = slots[s.c * stride];
+// Sums and products that are rounded one by one: the device compiler would
+// otherwise make a fused multiply-add of a product and the sum that reads it.
+KDN_HD float mulAlone(float a, float b) {
+#ifdef __CUDA_ARCH__
+	return __fmul_rn(a, b);
+#else
+	return a * b;
+#endif
+}
+KDN_HD float addAlone(float a, float b) {
+#ifdef __CUDA_ARCH__
+	return __fadd_rn(a, b);
+#else
+	return a + b;
+#endif
+}
+
+// world.h FormAxis: a coordinate's distance to a slab.
+KDN_HD float axisValue(float p, uint32_t side, const MarchParams& q) {
+	float u = addAlone(p, -q.v[0]);
+	u       = side == SideAbs ? fabsf(u) : u;
+	u       = side == SideNegative ? 0.0f - u : u;
+	return addAlone(addAlone(addAlone(u, -q.v[1]), q.v[2]), -q.v[3]);
+}
+
+// world.h FormSphere.
+KDN_HD float sphereValue(float px, float py, float pz, const MarchParams& q) {
+	const float x = addAlone(px, -q.v[0]), y = addAlone(py, -q.v[1]), z = addAlone(pz, -q.v[2]);
+	return addAlone(marchSqrt(fmaf(z, z, fmaf(x, x, mulAlone(y, y)))), -q.v[3]);
+}
+
+// world.h FormNorm over the values of its slots.
+KDN_HD float normValue(float a, float b, float c, float m, uint32_t flags, float e) {
+	const float p = flags & NormPositive0 ? fmaxf(a, 0.0f) : a;
+	const float q = flags & NormPositive1 ? fmaxf(b, 0.0f) : b;
+	const float r = flags & NormPositive2 ? fmaxf(c, 0.0f) : c;
+	float sum     = mulAlone(p, p);
+	sum           = flags & NormFused1 ? fmaf(q, q, sum) : addAlone(mulAlone(q, q), sum);
+	const float s = flags & NormFused2 ? fmaf(r, r, sum) : addAlone(mulAlone(r, r), sum);
+	float f       = marchSqrt(flags & NormThree ? s : sum);
+	if (flags & NormInside) {
+		if (flags & NormInsideMax) {
+			m = flags & NormThree ? (b < c ? c : b) : b;
+			m = a < m ? m : a;
+		}
+		f = addAlone(f, 0.0f < m ? 0.0f : m);
+	}
+	return addAlone(f, -e);
+}
+
+// One step of the march form (world.h MarchStep) and, of a fused step, its
+// parameters: r = post(form, w), with the post operations worked out
+// together and the step's picked, so the lanes of a warp on different posts
+// do not split; a rare step runs the reference operation.  Writes the result
+// to its slot.
+KDN_HD void marchStep(const MarchStep& s, const MarchParams& q, float* slots, uint32_t stride) {
 	float r;
 	if (s.op >= kMarchRare) {
+		slots[SlotImm * stride] = s.value;
+		const float a = slots[s.a * stride], b = slots[s.b * stride], c = slots[s.c * stride];
 		const float p[3] = { slots[SlotX * stride], slots[SlotY * stride], slots[SlotZ * stride] };
 		r                = stepValue(uint8_t(s.op - kMarchRare), a, b, c, s.value, p);
 	} else {
-		const float w = slots[s.w * stride];
-		const float f = fmaf(a, b, c);
-		const float q = fmaxf(f, 0.0f);
-		// the smooth minimum of radius r = value: min - max(r - |f - w|, 0)^2 * 0.25 / r
-		const float m = fmaxf(s.value - fabsf(f - w), 0.0f);
-		r             = f;
-		r             = s.op == PostSqrt ? marchSqrt(f) : r;
-		r             = s.op == PostAbs ? fabsf(f) : r;
-		r             = s.op == PostPosSq ? q * q : r;
-		r             = s.op == PostMin ? (w < f ? w : f) : r;
-		r             = s.op == PostMax ? (f < w ? w : f) : r;
-		r             = s.op == PostSminK ? fminf(f, w) - m * m * s.quarter : r;
+		const uint32_t form = s.op & kMarchFormMask, post = s.op & kMarchPostMask;
+		float f;
+		if (form == FormAxis) {
+			f = axisValue(slots[s.a * stride], s.flags, q);
+		} else if (form == FormSphere) {
+			f = sphereValue(slots[SlotX * stride], slots[SlotY * stride], slots[SlotZ * stride], q);
+		} else if (form == FormNorm) {
+			f = normValue(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride], slots[s.m * stride], s.flags, q.v[0]);
+		} else {
+			slots[SlotImm * stride] = s.value;
+			f                       = fmaf(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride]);
+		}
+		r = f;
+		if (post != PostNone) {
+			slots[SlotImm * stride] = s.value;
+			const float w = slots[s.w * stride];
+			const float p = fmaxf(f, 0.0f);
+			// the smooth minimum of radius r = value: min - max(r - |f - w|, 0)^2 * 0.25 / r
+			const float m = fmaxf(s.value - fabsf(f - w), 0.0f);
+			r             = post == PostSqrt ? marchSqrt(f) : r;
+			r             = post == PostAbs ? fabsf(f) : r;
+			r             = post == PostPosSq ? p * p : r;
+			r             = post == PostMin ? (w < f ? w : f) : r;
+			r             = post == PostMax ? (f < w ? w : f) : r;
+			r             = post == PostSminK ? fminf(f, w) - m * m * s.quarter : r;
+		}
 	}
 	slots[s.dst * stride] = r;
-	return r;
 }
+
+// The parameters of a fused step, in the unit after it.
+KDN_HD MarchParams paramsAt(const MarchStep* unit) {
+#ifdef __CUDA_ARCH__
+	const float4 v = *reinterpret_cast<const float4*>(unit);
+	return { { v.x, v.y, v.z, v.w } };
+#else
+	MarchParams q;
+	std::memcpy(&q, unit, sizeof q);
+	return q;
+#endif
+}
+
+// Whether a step is a fused one.
+KDN_HD bool fusedStep(const MarchStep& s) { return s.op < kMarchRare && (s.op & kMarchFormMask) != FormFma; }
 
 // One program at one point; slots is this thread's column base (stride
 // blockDim.x), with the constants set.  Returns the program's value.
 KDN_HD float evalSlots(const MarchStep* __restrict__ code, uint32_t count, uint32_t resultSlot, float* slots, uint32_t stride, const float p[3]) {
 	setPoint(slots, stride, p);
-	for (uint32_t i = 0; i < count; ++i) marchStep(code[i], slots, stride);
+	for (uint32_t i = 0; i < count; ++i) {
+		const MarchStep s = code[i];
+		MarchParams q {};
+		if (fusedStep(s)) q = paramsAt(code + ++i);
+		marchStep(s, q, slots, stride);
+	}
 	return slots[resultSlot * stride];
 }
 

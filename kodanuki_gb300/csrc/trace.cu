@@ -315,8 +315,10 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 		if (mode == Evaluating) {
 			for (uint32_t u = 0; u < kStepsPerTurn; ++u) {
 				const MarchStep s = next;
+				MarchParams q {};
+				if (fusedStep(s)) q = paramsAt(code + ++pc);
 				if (pc + 1 < length) next = code[pc + 1];
-				marchStep(s, slots, stride);
+				marchStep(s, q, slots, stride);
 				if (++pc == length) break;
 			}
 			if (pc == length) {
