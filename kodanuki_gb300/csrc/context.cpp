@@ -49,7 +49,7 @@ void Context::release() {
 	cudaSetDevice(device);
 	if (stream) cudaStreamSynchronize(stream);
 	releaseFrame();
-	for (DeviceBuffer* b : { &nodes, &leaves, &programs, &steps, &march, &ssa, &leafMaterial, &objectMaterial, &grid, &gridWalls, &extendRays, &extendHits, &extendStates, &counters, &l2, &denoiseScratch, &denoiseIo, &fetch, &upscale.samples, &upscale.axes, &sobolTables }) freeBuffer(*b);
+	for (DeviceBuffer* b : { &nodes, &leaves, &programs, &steps, &march, &ssa, &leafMaterial, &objectMaterial, &grid, &gridBricks, &fineWalls, &extendRays, &extendHits, &extendStates, &counters, &l2, &denoiseScratch, &denoiseIo, &fetch, &upscale.samples, &upscale.axes, &sobolTables }) freeBuffer(*b);
 	if (stream) cudaStreamDestroy(stream);
 	stream = nullptr;
 }
@@ -127,14 +127,19 @@ kdn_status Context::build(const BuildOptions& options) {
 	}
 	// the grid over the flat octree, for locating points
 	gridCells.clear();
+	bricks.clear();
 	walls.clear();
 	for (int a = 0; a < 3; ++a) {
 		lowerF[a] = float(regions[0].lower[a]);
 		sizeF[a]  = float(regions[0].size[a]);
 	}
 	if (!flat.nodes.empty()) {
-		gridCells = gridOf(flat, kGridLevel);
-		walls     = gridWallsOf(lowerF, sizeF, kGridLevel);
+		uint32_t deepest = kGridLevel;
+		for (const Cell& c : octree.cells) deepest = std::max(deepest, c.level);
+		fineLevel = fineLevelOf(lowerF, sizeF, std::min(deepest, kMostFine));
+		gridLevel = std::min(fineLevel, kGridLevel);
+		gridOf(flat, gridLevel, fineLevel, gridCells, bricks);
+		walls     = wallsOf(lowerF, sizeF, fineLevel);
 	}
 	// depth-first order of the cells, for kdn_world_cell
 	preorder.clear();
@@ -163,8 +168,9 @@ kdn_status Context::build(const BuildOptions& options) {
 	if ((s = upload(march, flat.march.data(), flat.march.size() * sizeof(MarchStep))) != KDN_OK) return s;
 	if ((s = upload(leafMaterial, leafMaterials.data(), leafMaterials.size() * sizeof(uint32_t))) != KDN_OK) return s;
 	if ((s = upload(objectMaterial, firstLeafMaterial.data(), firstLeafMaterial.size() * sizeof(uint32_t))) != KDN_OK) return s;
-	if ((s = upload(grid, gridCells.data(), gridCells.size() * sizeof(GridCell))) != KDN_OK) return s;
-	if ((s = upload(gridWalls, walls.data(), walls.size() * sizeof(float))) != KDN_OK) return s;
+	if ((s = upload(grid, gridCells.data(), gridCells.size() * sizeof(uint32_t))) != KDN_OK) return s;
+	if ((s = upload(gridBricks, bricks.data(), bricks.size() * sizeof(uint32_t))) != KDN_OK) return s;
+	if ((s = upload(fineWalls, walls.data(), walls.size() * sizeof(float))) != KDN_OK) return s;
 	if (!check(cudaStreamSynchronize(stream), "kdn_build upload")) return KDN_CUDA_ERROR;
 	world.nodes         = static_cast<const int32_t*>(nodes.ptr);
 	world.leaves        = static_cast<const GpuLeaf*>(leaves.ptr);
@@ -173,20 +179,26 @@ kdn_status Context::build(const BuildOptions& options) {
 	world.ssa           = static_cast<const SsaOps*>(ssa.ptr);
 	world.march         = static_cast<const MarchStep*>(march.ptr);
 	world.leaf_material = static_cast<const uint32_t*>(leafMaterial.ptr);
-	world.grid          = static_cast<const GridCell*>(grid.ptr);
-	world.gridWalls     = static_cast<const float*>(gridWalls.ptr);
-	world.gridLevel     = kGridLevel;
-	for (int a = 0; a < 3; ++a) {
-		world.lower[a] = float(regions[0].lower[a]);
-		world.size[a]  = float(regions[0].size[a]);
-		world.gridScale[a] = float(double(1u << kGridLevel) / double(world.size[a]));
-	}
+	world.grid          = static_cast<const uint32_t*>(grid.ptr);
+	world.bricks        = static_cast<const uint32_t*>(gridBricks.ptr);
+	world.walls         = static_cast<const float*>(fineWalls.ptr);
+	setLocating(world);
 	world.leaf_count     = uint32_t(flat.leaves.size());
 	world.material_count = uint32_t(block<kdn_material>("looks.materials").size());
 	world.marchSlots     = 1;
 	for (const GpuProgram& g : flat.programs) world.marchSlots = std::max<uint32_t>(world.marchSlots, g.marchSlots);
 	built                = true;
 	return KDN_OK;
+}
+
+void Context::setLocating(DeviceWorld& to) const {
+	to.gridLevel = gridLevel;
+	to.fineLevel = fineLevel;
+	for (int a = 0; a < 3; ++a) {
+		to.lower[a] = lowerF[a];
+		to.size[a]  = sizeF[a];
+	}
+	placeScale(lowerF, sizeF, fineLevel, to.scale, to.bias);
 }
 
 int64_t Context::preorderCell(uint64_t i) const {

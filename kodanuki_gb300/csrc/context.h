@@ -57,12 +57,13 @@ struct Context {
 	Octree octree;
 	FlatWorld flat;
 	std::string flatError; // why a host-only context has no device layout
-	std::vector<GridCell> gridCells; // the grid over the flat octree (world.h GridCell)
-	std::vector<float> walls;        // its walls per axis
+	std::vector<uint32_t> gridCells, bricks; // the grid over the flat octree and its bricks (world.h kEntryLeaf)
+	std::vector<float> walls;       // its walls per axis down to fineLevel
+	uint32_t fineLevel = 0, gridLevel = 0;
 	float lowerF[3] = {}, sizeF[3] = {};
 	std::vector<int64_t> preorder; // cell index of each depth-first position
 	DeviceWorld world {};
-	DeviceBuffer nodes, leaves, programs, steps, march, ssa, leafMaterial, objectMaterial, grid, gridWalls;
+	DeviceBuffer nodes, leaves, programs, steps, march, ssa, leafMaterial, objectMaterial, grid, gridBricks, fineWalls;
 	DeviceBuffer extendRays, extendHits, extendStates, counters, l2;
 	DeviceBuffer denoiseScratch, denoiseIo, fetch;
 	UpscaleScratch upscale; // kdn_upscale_device's
@@ -92,6 +93,7 @@ struct Context {
 	bool has(const char* name) const { return blocks.count(name) != 0; }
 	kdn_status build(const BuildOptions& options);
 	int64_t preorderCell(uint64_t i) const;
+	void setLocating(DeviceWorld& to) const; // how points are located, but for the tables' pointers
 	kdn_status extend(const kdn_ray* rays, uint32_t n, kdn_hit* hits, cudaStream_t on);
 	kdn_status flushL2();
 	void releaseFrame();

@@ -1,5 +1,5 @@
-// Locating the octree leaf a point lies in (the trace kernel's descent),
-// for the device and, to check it, the host.
+// Locating the octree leaf a point lies in, for the device and, to check it,
+// the host.
 #pragma once
 
 #include "program.cuh"
@@ -17,70 +17,45 @@ KDN_HD T loadOnce(const T* p) {
 #endif
 }
 
-struct Located {
-	uint32_t leaf;
-	float lo[3], hi[3];
-};
-
-KDN_HD Located locate(const DeviceWorld& w, const float p[3]) {
-	Located l;
-	int32_t node;
-	if (w.grid != nullptr) {
-		// the grid cell: an estimate from the coordinates, set right against
-		// the walls (the descent's own midpoints: a point on a wall goes up)
-		const int n = 1 << w.gridLevel;
-		int cell[3];
-		for (int a = 0; a < 3; ++a) {
-			const float* walls = w.gridWalls + a * (n + 1);
-			int i              = int(fminf(fmaxf((p[a] - w.lower[a]) * w.gridScale[a], 0.0f), float(n - 1)));
-			if (i > 0 && p[a] < loadOnce(walls + i)) --i;
-			else if (i < n - 1 && p[a] >= loadOnce(walls + i + 1)) ++i;
-			cell[a] = i;
-		}
-		const GridCell g = w.grid[(size_t(cell[2]) * n + cell[1]) * n + cell[0]];
-		node             = g.node;
-		// the box of the cell's level (a leaf above the grid's level is bigger)
-		const int shift = int(w.gridLevel) - int(g.level);
-		for (int a = 0; a < 3; ++a) {
-			const float* walls = w.gridWalls + a * (n + 1);
-			const int i0       = (cell[a] >> shift) << shift;
-			l.lo[a]            = loadOnce(walls + i0);
-			l.hi[a]            = loadOnce(walls + i0 + (1 << shift));
-		}
-	} else {
-		for (int a = 0; a < 3; ++a) {
-			l.lo[a] = w.lower[a];
-			l.hi[a] = w.lower[a] + w.size[a];
-		}
-		node = loadOnce(&w.nodes[0]);
-	}
-	uint32_t at = 0;
-	for (int depth = 0; depth < 30 && node >= 0; ++depth) {
-		int o = 0;
-		for (int a = 0; a < 3; ++a) {
-			const float mid = 0.5f * (l.lo[a] + l.hi[a]);
-			if (p[a] >= mid) {
-				o |= 1 << a;
-				l.lo[a] = mid;
-			} else {
-				l.hi[a] = mid;
-			}
-		}
-		at   = uint32_t(node) + uint32_t(o);
-		node = loadOnce(&w.nodes[at]);
-	}
-	l.leaf = uint32_t(~node);
-	return l;
+// The place below a coordinate's estimate; not a number is place 0.
+KDN_HD int placeBelow(float x) {
+#ifdef __CUDA_ARCH__
+	return __float2int_rd(x);
+#else
+	return x >= 2147483648.0f ? 0x7FFFFFFF : x >= -2147483648.0f ? int(floorf(x)) : x < 0.0f ? int(0x80000000) : 0;
+#endif
 }
 
-// The descent from the root alone, the reference for locate()'s grid.
-KDN_HD uint32_t descendFromRoot(const DeviceWorld& w, const float p[3]) {
-	float lo[3], hi[3];
+// A point's place among the tabled walls, the boundary's past the region.
+KDN_HD void placeOf(const DeviceWorld& w, const float p[3], int place[3]) {
+	const int n = 1 << w.fineLevel;
 	for (int a = 0; a < 3; ++a) {
-		lo[a] = w.lower[a];
-		hi[a] = w.lower[a] + w.size[a];
+		int i = placeBelow(fmaf(p[a], w.scale[a], w.bias[a]));
+		i     = i < 0 ? 0 : i > n - 1 ? n - 1 : i;
+		if (p[a] >= loadOnce(w.walls + a * (n + 1) + i + 1)) ++i;
+		place[a] = i > n - 1 ? n - 1 : i;
 	}
-	int32_t node = w.nodes[0];
+}
+
+// The entry at a place (world.h kEntryLeaf): a leaf, or below the finest
+// tabled level an inner node.
+KDN_HD uint32_t entryAt(const DeviceWorld& w, const int place[3]) {
+	uint32_t s     = w.fineLevel - w.gridLevel;
+	uint32_t entry = loadOnce(w.grid + ((size_t(place[2] >> s) << w.gridLevel | size_t(place[1] >> s)) << w.gridLevel | size_t(place[0] >> s)));
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+	while (!(entry & kEntryLeaf) && s > 0) {
+		// the place's next two bits an axis (the last one alone where one is left)
+		const int mask = s > 1 ? 3 : 1;
+		s -= s > 1 ? 2 : 1;
+		entry = loadOnce(w.bricks + size_t(entry) * kBrick + ((place[0] >> s & mask) | (place[1] >> s & mask) << 2 | (place[2] >> s & mask) << 4));
+	}
+	return entry;
+}
+
+// The leaf below an inner node of the finest tabled level, and its box.
+KDN_HD int32_t descend(const DeviceWorld& w, const float p[3], int32_t node, float lo[3], float hi[3]) {
 	for (int depth = 0; depth < 30 && node >= 0; ++depth) {
 		int o = 0;
 		for (int a = 0; a < 3; ++a) {
@@ -92,9 +67,34 @@ KDN_HD uint32_t descendFromRoot(const DeviceWorld& w, const float p[3]) {
 				hi[a] = mid;
 			}
 		}
-		node = w.nodes[uint32_t(node) + uint32_t(o)];
+		node = loadOnce(w.nodes + node + o);
 	}
-	return uint32_t(~node);
+	return node;
+}
+
+// The leaf a point lies in.
+KDN_HD uint32_t locate(const DeviceWorld& w, const float p[3]) {
+	int place[3];
+	placeOf(w, p, place);
+	const uint32_t entry = entryAt(w, place);
+	if (entry & kEntryLeaf) return entry & kEntryIndex;
+	float lo[3], hi[3];
+	for (int a = 0; a < 3; ++a) {
+		const float* walls = w.walls + a * ((1 << w.fineLevel) + 1) + place[a];
+		lo[a]              = loadOnce(walls);
+		hi[a]              = loadOnce(walls + 1);
+	}
+	return uint32_t(~descend(w, p, int32_t(entry), lo, hi));
+}
+
+// The descent from the root alone, the reference for locate().
+KDN_HD uint32_t descendFromRoot(const DeviceWorld& w, const float p[3]) {
+	float lo[3], hi[3];
+	for (int a = 0; a < 3; ++a) {
+		lo[a] = w.lower[a];
+		hi[a] = w.lower[a] + w.size[a];
+	}
+	return uint32_t(~descend(w, p, loadOnce(&w.nodes[0]), lo, hi));
 }
 
 } // namespace kdn

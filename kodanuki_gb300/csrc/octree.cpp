@@ -560,12 +560,14 @@ struct Node {
 	// how far an axis has come (the terms taken so far), and the single steps
 	// it stands for
 	uint8_t form  = FormFma, flags = 0;
-	Operand m;             // FormNorm: the inside term
+	bool inside = false;   // FormNorm: an inside term, m
+	Operand m;
 	float params[4] = { 0.0f, 0.0f, -0.0f, 0.0f };
 	uint8_t stage = 0;     // FormAxis: 0 none, 1 c, 2 a side, 3 h, 4 r, 5 e; else 1 once e is taken
 	uint32_t took = 1;
-	Operand single;        // FormAxis of one step: that step's a and post
-	uint8_t singlePost = PostNone;
+	// FormPrimitive: its flags, its terms (axis and side), their c, h and r (params[3] is e)
+	uint8_t kind = 0, terms[3] = { 0, 0, 0 };
+	float centre[3] = { 0.0f, 0.0f, 0.0f }, half[3] = { 0.0f, 0.0f, 0.0f }, round = -0.0f;
 };
 
 // sdf/program.cpp:57 runStep in double, for steps of constants alone.
@@ -642,17 +644,15 @@ struct Readers {
 bool readsW(const Node& n) { return n.post == PostMin || n.post == PostMax || n.post == PostSminK; }
 template <typename F>
 void eachOperand(const Node& n, const F& read) {
-	if (n.form == FormSphere) {
-		if (readsW(n)) read(n.w);
-		return;
-	}
-	read(n.a);
-	if (n.form != FormAxis) {
-		read(n.b);
-		read(n.c);
+	if (n.form != FormPrimitive) {
+		read(n.a);
+		if (n.form != FormAxis && n.form != FormRepeat) {
+			read(n.b);
+			read(n.c);
+		}
+		if (n.form == FormNorm && n.inside) read(n.m);
 	}
 	if (readsW(n)) read(n.w);
-	if (n.form == FormNorm) read(n.m);
 }
 Readers readersOf(const std::vector<Node>& nodes, uint32_t result) {
 	Readers r;
@@ -747,8 +747,6 @@ struct Fusing {
 		const Sum sum = sumWith(n, x, value);
 		Node f        = n;
 		f.form        = FormAxis;
-		f.single      = n.a;
-		f.singlePost  = n.post;
 		if (sum != NoSum && point(x)) {
 			f.a         = x;
 			f.params[0] = sum == Plus ? -float(value) : float(value);
@@ -800,6 +798,31 @@ struct Fusing {
 		} else {
 			return;
 		}
+		n = f;
+	}
+
+	// x - s * floor(x / s + o)
+	void repeat(Node& n) {
+		if (n.rare || n.form != FormFma || n.post != PostNone || !is(n.b, SlotMinusOne) || n.c.kind != Operand::Node) return;
+		const Node* scaled = only(n.a);
+		if (!scaled || scaled->form != FormFma || scaled->post != PostNone || scaled->a.kind != Operand::Immediate || !is(scaled->c, SlotZero)) return;
+		const auto rareOnly = [&](const Operand& o, uint8_t op) -> const Node* {
+			return o.kind == Operand::Node && reads.uses[o.node] == 1 && nodes[o.node].rare && nodes[o.node].refOp == op ? &nodes[o.node] : nullptr;
+		};
+		const Node* whole = rareOnly(scaled->b, OpFloor);
+		if (!whole) return;
+		const Node* moved = only(whole->a);
+		Operand x;
+		double offset = 0.0;
+		if (!moved || moved->post != PostNone || sumWith(*moved, x, offset) != Plus) return;
+		const Node* over = rareOnly(x, OpDivide);
+		if (!over || !same(over->a, n.c) || over->b.kind != Operand::Immediate || over->b.value != scaled->a.value) return;
+		Node f   = n;
+		f.form   = FormRepeat;
+		f.a      = n.c;
+		f.radius = scaled->a.value;
+		f.params[0] = float(offset);
+		f.took += scaled->took + whole->took + moved->took + over->took;
 		n = f;
 	}
 
@@ -873,39 +896,23 @@ struct Fusing {
 		Node f  = n;
 		f.form  = FormNorm;
 		f.post  = PostNone;
-		f.flags = uint8_t(t.size() == 3 ? NormThree : 0);
-		f.c     = Operand();
+		f.flags = 0;
+		f.c     = f.b = Operand();
 		Operand* slots[3] = { &f.a, &f.b, &f.c };
 		for (size_t k = 0; k < t.size(); ++k) {
 			if (t[k].x.kind == Operand::Immediate) return;
 			*slots[k] = t[k].x;
-			if (t[k].positive) f.flags |= uint8_t(NormPositive0 << k);
-			if (t[k].fused) f.flags |= uint8_t(k == 1 ? NormFused1 : NormFused2);
+			f.flags |= uint8_t(SumHas0 << k);
+			if (t[k].positive) f.flags |= uint8_t(SumPositive0 << k);
+			if (t[k].fused) f.flags |= uint8_t(k == 1 ? SumFused1 : SumFused2);
 			f.took += t[k].took;
 		}
 		for (const Term& k : t) {
-			if (k.strip) k.strip->post = k.strip->singlePost = PostNone;
+			if (k.strip) k.strip->post = PostNone;
 		}
 		f.params[0] = 0.0f;
 		f.stage     = 0;
-		// a point's distance to a centre: y first, then x and z by fused multiply-adds
-		const uint8_t order[3] = { SlotY, SlotX, SlotZ };
-		bool sphere            = f.flags == (NormThree | NormFused1 | NormFused2);
-		const Node* part[3]    = {};
-		for (int k = 0; k < 3 && sphere; ++k) {
-			part[k] = only(*slots[k], 2);
-			sphere  = part[k] && part[k]->form == FormAxis && part[k]->stage == 1 && part[k]->post == PostNone && is(part[k]->a, order[k]);
-		}
-		if (sphere) {
-			f.form  = FormSphere;
-			f.flags = 0;
-			f.params[0] = part[1]->params[0];
-			f.params[1] = part[0]->params[0];
-			f.params[2] = part[2]->params[0];
-			f.params[3] = 0.0f;
-			for (const Node* k : part) f.took += k->took;
-		}
-		n = f;
+		n           = f;
 	}
 	// the inside term of a box, and the rounding or the radius
 	void around(Node& n) {
@@ -913,12 +920,12 @@ struct Fusing {
 		double value = 0.0;
 		if (sumWith(n, x, value) == Minus) {
 			const Node* b = only(x);
-			if (!b || (b->form != FormNorm && b->form != FormSphere) || b->post != PostNone || b->stage != 0) return;
-			Node f  = *b;
-			f.post  = n.post;
-			f.w     = n.w;
+			if (!b || (b->form != FormNorm && b->form != FormPrimitive) || b->post != PostNone || b->stage != 0) return;
+			Node f   = *b;
+			f.post   = n.post;
+			f.w      = n.w;
 			f.radius = n.radius;
-			f.stage = 1;
+			f.stage  = 1;
 			f.took += n.took;
 			f.params[b->form == FormNorm ? 0 : 3] = float(value);
 			n = f;
@@ -928,40 +935,185 @@ struct Fusing {
 		for (int k = 0; k < 2; ++k) {
 			const Node* b = only(k == 0 ? n.a : n.c);
 			const Node* m = only(k == 0 ? n.c : n.a);
-			if (!b || !m || b->form != FormNorm || b->post != PostNone || b->stage != 0 || (b->flags & NormInside)) continue;
 			Operand h;
-			if (m->post != PostMin || m->w.kind != Operand::Immediate || m->w.value != 0.0 || !copyOf(*m, h)) continue;
-			Node f = *b;
-			f.post = n.post;
-			f.w    = n.w;
+			if (!b || !m || b->form != FormNorm || b->post != PostNone || b->stage != 0 || b->inside || !leastOfZero(*m, h)) continue;
+			Node f   = *b;
+			f.post   = n.post;
+			f.w      = n.w;
 			f.radius = n.radius;
-			f.flags |= NormInside;
-			f.m = h;
+			f.inside = true;
+			f.m      = h;
 			f.took += n.took + m->took;
-			// the inside term the terms' own maximum: max(a, max(b, c)), or max(a, b)
-			Operand p, q;
-			const Node* outer = only(h);
-			if (outer && outer->post == PostMax && copyOf(*outer, p) && same(p, f.a)) {
-				if (!(f.flags & NormThree) && same(outer->w, f.b)) {
-					f.flags |= NormInsideMax;
-					f.took += outer->took;
-				} else if (const Node* inner = only(outer->w); inner && (f.flags & NormThree) && inner->post == PostMax && copyOf(*inner, q) && same(q, f.b) && same(inner->w, f.c)) {
-					f.flags |= NormInsideMax;
-					f.took += outer->took + inner->took;
-				}
-				if (f.flags & NormInsideMax) f.m = Operand();
-			}
 			n = f;
 			return;
 		}
 	}
+	// min(x, 0) and max(x, 0)
+	static bool withZero(const Node& n, uint8_t post, Operand& x) { return n.post == post && n.w.kind == Operand::Immediate && n.w.value == 0.0 && copyOf(n, x); }
+	static bool leastOfZero(const Node& n, Operand& x) { return withZero(n, PostMin, x); }
+
+	// ---- primitives: a root or a slab over slabs of the point alone ----
+
+	// the slabs a primitive is made of, each with how often it reads them
+	struct Slabs {
+		std::vector<uint32_t> nodes, reads;
+		bool add(const Operand& o, const std::vector<Node>& all, uint32_t& place, uint8_t post = PostNone) {
+			if (o.kind != Operand::Node || all[o.node].rare || all[o.node].form != FormAxis || all[o.node].stage > 4 || all[o.node].post != post) return false;
+			for (place = 0; place < nodes.size(); ++place) {
+				if (nodes[place] == o.node) break;
+			}
+			if (place == nodes.size()) {
+				if (nodes.size() == 3) return false;
+				nodes.push_back(o.node);
+				reads.push_back(0);
+			}
+			reads[place] += 1;
+			return true;
+		}
+	};
+	// an inside term's slabs in the order of its maxima: max(t0, t1), or max(t0, max(t1, t2))
+	bool maxima(const Operand& o, Slabs& s) const {
+		uint32_t place = 0;
+		Operand at     = o;
+		for (uint32_t depth = 0; depth < 2; ++depth) {
+			const Node* n = only(at);
+			if (!n || n->post != PostMax) return false;
+			Operand f;
+			// a slab that makes the maximum itself, or a maximum of its own
+			const bool made = n->form == FormAxis;
+			if (!made && !copyOf(*n, f)) return false;
+			if (!s.add(made ? at : f, nodes, place, made ? PostMax : PostNone) || place != depth) return false;
+			at               = n->w;
+			const Node* next = only(at);
+			if (!next || next->post != PostMax) return s.add(at, nodes, place) && place == depth + 1;
+		}
+		return false;
+	}
+	// the terms of a primitive from its slabs, where they allow it: no other
+	// reader, no post but the maximum it makes, and one r among them
+	bool termed(Node& f, const Slabs& s) const {
+		for (size_t k = 0; k < s.nodes.size(); ++k) {
+			const Node& x = nodes[s.nodes[k]];
+			if (reads.uses[s.nodes[k]] != s.reads[k]) return false;
+			if (k > 0 && std::memcmp(&x.params[2], &f.round, sizeof f.round) != 0) return false;
+			f.round     = x.params[2];
+			f.centre[k] = x.params[0];
+			f.half[k]   = x.params[1];
+			f.terms[k]  = uint8_t(x.a.slot - SlotX) | uint8_t(x.flags << kTermSideShift);
+			f.took += x.took;
+		}
+		return true;
+	}
+	void primitive(Node& n) {
+		if (n.rare) return;
+		if (n.form == FormAxis) { // the slab itself
+			Node f   = n;
+			f.form   = FormPrimitive;
+			f.kind   = PrimPlain;
+			f.flags  = 0;
+			f.stage  = 1;
+			f.round     = n.params[2];
+			f.centre[0] = n.params[0];
+			f.half[0]   = n.params[1];
+			f.terms[0]  = uint8_t(n.a.slot - SlotX) | uint8_t(n.flags << kTermSideShift);
+			n = f;
+			return;
+		}
+		if (n.form == FormNorm) {
+			Slabs s;
+			if (n.inside && !maxima(n.m, s)) return;
+			const Operand* slots[3] = { &n.a, &n.b, &n.c };
+			Node f  = n;
+			f.form  = FormPrimitive;
+			f.flags = 0;
+			f.kind  = uint8_t(n.inside ? PrimInside | (s.nodes.size() == 3 ? PrimThird : 0) : 0);
+			for (int k = 0; k < 3; ++k) {
+				uint32_t place = 0;
+				if (!(n.flags & SumHas0 << k)) continue;
+				if (!s.add(*slots[k], nodes, place) || (f.flags & SumHas0 << place)) return;
+				// a sum adds its terms in their order, but the first two in either
+				// where neither is a fused multiply-add, and any two alone
+				const bool turned = place != uint32_t(k);
+				const bool three  = n.flags & SumHas2;
+				if (turned && ((n.flags & (SumFused1 | SumFused2)) || (three && (k == 2 || place == 2)))) return;
+				f.flags |= uint8_t(SumHas0 << place);
+				if (n.flags & SumPositive0 << k) f.flags |= uint8_t(SumPositive0 << place);
+			}
+			f.flags |= uint8_t(n.flags & (SumFused1 | SumFused2));
+			f.params[3] = n.params[0];
+			if (termed(f, s)) n = f;
+			return;
+		}
+		if (n.form != FormFma || !is(n.b, SlotOne) || n.post != PostNone) {
+			joinedBy(n);
+			return;
+		}
+		// max(q, 0) + min(m, 0), m a maximum that q is in
+		for (int k = 0; k < 2; ++k) {
+			const Node* most = only(k == 0 ? n.a : n.c);
+			const Node* least = only(k == 0 ? n.c : n.a);
+			Operand q, m;
+			Slabs s;
+			uint32_t place = 0;
+			if (!most || !least || !withZero(*most, PostMax, q) || !leastOfZero(*least, m) || !maxima(m, s) || s.nodes.size() < 2) continue;
+			const size_t slabs = s.nodes.size();
+			if (!s.add(q, nodes, place) || s.nodes.size() != slabs) continue;
+			Node f  = n;
+			f.form  = FormPrimitive;
+			f.flags = uint8_t(SumHas0 << place);
+			f.kind  = uint8_t(PrimSingle | PrimInside | (slabs == 3 ? PrimThird : 0));
+			f.stage = 0;
+			f.params[3] = 0.0f;
+			f.took += most->took + least->took;
+			if (termed(f, s)) {
+				n = f;
+				return;
+			}
+		}
+		joinedBy(n);
+	}
+	// a post operation of its own on a primitive: the primitive's
+	void joinedBy(Node& n) {
+		Operand x;
+		if (!readsW(n) || !copyOf(n, x)) return;
+		const Node* b = only(x);
+		Operand w     = n.w;
+		if ((!b || b->form != FormPrimitive || b->post != PostNone) && n.post == PostSminK) { // either way about
+			b = only(n.w);
+			w = x;
+		}
+		if (!b || b->form != FormPrimitive || b->post != PostNone) return;
+		Node f   = *b;
+		f.post   = n.post;
+		f.w      = w;
+		f.radius = n.radius;
+		f.took += n.took;
+		n = f;
+	}
+
 	void run() {
 		for (size_t j = 0; j < nodes.size(); ++j) {
 			if (!reads.live[j] || nodes[j].rare) continue;
 			joined(nodes[j]);
+			repeat(nodes[j]);
 			axis(nodes[j]);
 			norm(nodes[j]);
 			around(nodes[j]);
+		}
+	}
+	void runPrimitives() {
+		for (size_t j = 0; j < nodes.size(); ++j) {
+			if (!reads.live[j] || nodes[j].form == FormAxis) continue; // a slab waits for the root that reads it
+			primitive(nodes[j]);
+			around(nodes[j]);
+		}
+	}
+	// the slabs no root took
+	void runSlabs() {
+		for (size_t j = 0; j < nodes.size(); ++j) {
+			if (!reads.live[j]) continue;
+			if (nodes[j].form == FormAxis) primitive(nodes[j]);
+			else if (nodes[j].form == FormFma && !nodes[j].rare) joinedBy(nodes[j]);
 		}
 	}
 };
@@ -1154,6 +1306,8 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 	const Readers single = readersOf(L.nodes, result.node);
 	out.marchSteps       = uint16_t(std::count(single.live.begin(), single.live.end(), 1));
 	Fusing { L.nodes, single }.run();
+	Fusing { L.nodes, readersOf(L.nodes, result.node) }.runPrimitives();
+	Fusing { L.nodes, readersOf(L.nodes, result.node) }.runSlabs();
 	// the steps the result needs, and each one's last reader
 	const uint32_t m                = uint32_t(L.nodes.size());
 	const std::vector<uint8_t> live = readersOf(L.nodes, result.node).live;
@@ -1165,6 +1319,19 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 		});
 	}
 	lastRead[result.node] = m;
+	// which steps' results are read from their slots: all but those that only
+	// the next step reads, a primitive as its post operation's w
+	std::vector<uint8_t> stored(m, 0);
+	uint32_t before = 0xFFFFFFFFu;
+	for (uint32_t j = 0; j < m; ++j) {
+		if (!live[j]) continue;
+		const Node& x = L.nodes[j];
+		eachOperand(x, [&](const Operand& o) {
+			if (o.kind == Operand::Node && !(x.form == FormPrimitive && o.node == before)) stored[o.node] = 1;
+		});
+		before = j;
+	}
+	before = 0xFFFFFFFFu;
 	std::vector<uint8_t> slot(m, 0);
 	std::vector<uint8_t> freeSlots;
 	uint32_t used = kMarchFirstSlot;
@@ -1173,13 +1340,6 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 	for (uint32_t j = 0; j < m; ++j) {
 		if (!live[j]) continue;
 		Node& x = L.nodes[j];
-		// an axis of one term costs no less fused than single, but where it is the whole program
-		if (x.form == FormAxis && x.took == 1 && j != result.node) {
-			x.form = FormFma;
-			x.a    = x.single;
-			x.post = x.singlePost;
-		}
-		const bool fused = x.form != FormFma;
 		const bool usesW = readsW(x);
 		MarchStep g      = {};
 		g.op             = x.rare ? uint8_t(kMarchRare + x.refOp) : uint8_t(x.form + x.post);
@@ -1192,16 +1352,28 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 			}
 			return o.slot;
 		};
-		if (x.form != FormSphere) g.a = slotOf(x.a);
-		if (x.form == FormFma || x.form == FormNorm) {
-			g.b = slotOf(x.b);
-			g.c = slotOf(x.c);
+		const bool sized = x.form == FormPrimitive && !(x.half[0] == 0.0f && x.half[1] == 0.0f && x.half[2] == 0.0f && x.round == 0.0f && std::signbit(x.round));
+		if (x.form == FormPrimitive) {
+			g.a     = x.terms[0];
+			g.b     = x.terms[1];
+			g.c     = x.terms[2];
+			g.flags = x.flags;
+			g.m     = uint8_t(x.kind | (sized ? PrimSized : 0) | (usesW && x.w.kind == Operand::Node && x.w.node == before ? PrimPrevious : 0) | (stored[j] ? PrimStored : 0));
+		} else {
+			g.a = slotOf(x.a);
+			if (x.form != FormRepeat) {
+				g.b = slotOf(x.b);
+				g.c = slotOf(x.c);
+			}
+			if (x.form == FormNorm) {
+				g.m     = x.inside ? slotOf(x.m) : kNoInside;
+				g.flags = x.flags;
+			}
 		}
-		if (x.form == FormNorm) g.m = slotOf(x.m);
-		if (fused) g.flags = x.flags;
+		before    = j;
 		g.w       = usesW ? slotOf(x.w) : uint8_t(SlotZero);
-		g.value   = float(x.post == PostSminK ? x.radius : immValue);
-		g.quarter = x.post == PostSminK ? float(0.25 / x.radius) : 0.0f;
+		g.value   = float(x.post == PostSminK || x.form == FormRepeat ? x.radius : immValue);
+		g.quarter = x.post == PostSminK ? float(0.25 / x.radius) : x.form == FormRepeat ? x.params[0] : 0.0f;
 		// free the slots read here for the last time (each value once)
 		std::vector<uint32_t> freed;
 		eachOperand(x, [&](const Operand& o) {
@@ -1220,17 +1392,19 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 		g.dst = slot[j];
 		steps.push_back(g);
 		++kept;
-		if (fused) {
-			MarchParams q;
-			std::copy(x.params, x.params + 4, q.v);
-			MarchStep unit;
-			std::memcpy(&unit, &q, sizeof unit);
-			steps.push_back(unit);
+		const auto unit = [&](float v0, float v1, float v2, float v3) {
+			const float v[4] = { v0, v1, v2, v3 };
+			MarchStep u;
+			static_assert(sizeof u == sizeof v, "parameters are one unit");
+			std::memcpy(&u, v, sizeof u);
+			steps.push_back(u);
 			++kept;
-		}
+		};
+		if (x.form == FormPrimitive) unit(x.centre[0], x.centre[1], x.centre[2], x.params[3]);
+		if (sized) unit(x.half[0], x.half[1], x.half[2], x.round);
+		if (x.form == FormNorm) unit(x.params[0], 0.0f, 0.0f, 0.0f);
 	}
 	out.marchCount = uint16_t(kept);
-	out.marchSlot  = slot[result.node];
 	out.marchSlots = uint8_t(used);
 	return "";
 }
@@ -1329,21 +1503,36 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 			continue;
 		}
 		GpuLeaf leaf   = {};
-		leaf.occupancy = c.occupancy;
-		leaf.count     = uint16_t(c.programs.size());
+		leaf.count     = uint8_t(c.programs.size());
 		leaf.first     = uint32_t(flat.programs.size());
-		uint32_t slots = 1;
-		for (size_t k = 0; k < c.programs.size(); ++k) {
-			const GpuProgram& g = programs[named[at++]];
-			slots               = std::max<uint32_t>(slots, g.slots);
-			flat.programs.push_back(g);
-		}
-		leaf.slots = uint8_t(slots);
-		if (leaf.count > 0) {
+		for (size_t k = 0; k < c.programs.size(); ++k) flat.programs.push_back(programs[named[at++]]);
+		leaf.shape     = ShapePrograms;
+		if (c.occupancy == Empty || leaf.count == 0) {
+			leaf.shape     = ShapeEmpty;
+			leaf.params[0] = -std::numeric_limits<float>::infinity();
+			leaf.params[2] = -0.0f;
+		} else {
 			const GpuProgram& g = flat.programs[leaf.first];
 			leaf.march          = g.march;
 			leaf.marchCount     = g.marchCount;
-			leaf.marchSlot      = g.marchSlot;
+			leaf.marchSteps     = g.marchSteps;
+			const MarchStep& s  = flat.march[g.march];
+			std::memcpy(leaf.params, &s, sizeof leaf.params);
+			if (leaf.count == 1 && s.op == FormPrimitive && g.marchCount == (s.m & PrimSized ? 3 : 2)) {
+				float c[4], h[4] = { 0.0f, 0.0f, 0.0f, -0.0f };
+				std::memcpy(c, &flat.march[g.march + 1], sizeof c);
+				if (s.m & PrimSized) std::memcpy(h, &flat.march[g.march + 2], sizeof h);
+				const uint8_t all = SumHas0 | SumHas1 | SumHas2 | SumFused1 | SumFused2;
+				if (s.m & PrimPlain) {
+					const float q[4] = { c[0], h[0], h[3], c[3] };
+					std::copy(q, q + 4, leaf.params);
+					leaf.shape = uint8_t(ShapeAxis | (s.a & 3) << kShapeAxisShift | (s.a >> kTermSideShift) << kShapeSideShift);
+				} else if (s.m == 0 && s.flags == all && s.a == 1 && s.b == 0 && s.c == 2) { // y, x, z
+					const float q[4] = { c[1], c[0], c[2], c[3] };
+					std::copy(q, q + 4, leaf.params);
+					leaf.shape = ShapeSphere;
+				}
+			}
 		}
 		flat.nodes[i] = ~int32_t(flat.leaves.size());
 		flat.leaves.push_back(leaf);
@@ -1351,7 +1540,7 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 	return "";
 }
 
-std::vector<float> gridWallsOf(const float lower[3], const float size[3], uint32_t level) {
+std::vector<float> wallsOf(const float lower[3], const float size[3], uint32_t level) {
 	const uint32_t n = 1u << level;
 	std::vector<float> walls(3 * size_t(n + 1));
 	for (int a = 0; a < 3; ++a) {
@@ -1368,25 +1557,89 @@ std::vector<float> gridWallsOf(const float lower[3], const float size[3], uint32
 	return walls;
 }
 
-std::vector<GridCell> gridOf(const FlatWorld& flat, uint32_t level) {
-	const uint32_t side = 1u << level;
-	std::vector<GridCell> grid(size_t(side) * side * side);
-	for (uint32_t z = 0; z < side; ++z) {
-		for (uint32_t y = 0; y < side; ++y) {
-			for (uint32_t x = 0; x < side; ++x) {
-				int32_t node = flat.nodes[0];
-				uint32_t at  = 0;
-				for (; at < level && node >= 0; ++at) {
-					// the child of the cell holding (x, y, z): its bit at this level per axis
-					const uint32_t shift = level - 1 - at;
-					const uint32_t o     = ((x >> shift) & 1u) | (((y >> shift) & 1u) << 1) | (((z >> shift) & 1u) << 2);
-					node                 = flat.nodes[size_t(node) + o];
-				}
-				grid[(size_t(z) * side + y) * side + x] = GridCell { node, at };
+void placeScale(const float lower[3], const float size[3], uint32_t level, float scale[3], float bias[3]) {
+	for (int a = 0; a < 3; ++a) {
+		scale[a] = float(double(1u << level) / double(size[a]));
+		bias[a]  = float(-double(lower[a]) * double(scale[a]) - 0.25);
+	}
+}
+
+uint32_t fineLevelOf(const float lower[3], const float size[3], uint32_t most) {
+	for (uint32_t level = most; level > 0; --level) {
+		const uint32_t n               = 1u << level;
+		const std::vector<float> walls = wallsOf(lower, size, level);
+		float scale[3], bias[3];
+		placeScale(lower, size, level, scale, bias);
+		// the estimate never falls with the coordinate, so a place's ends tell
+		// for all of it: no more than one low at its first point, and not above
+		// it at its last
+		bool holds = true;
+		for (int a = 0; a < 3 && holds; ++a) {
+			const float* w = walls.data() + size_t(a) * (n + 1);
+			for (uint32_t i = 0; i < n && holds; ++i) {
+				const float last = std::nextafter(w[i + 1], w[i]);
+				holds            = w[i] < w[i + 1] && std::floor(std::fma(w[i], scale[a], bias[a])) >= float(i) - 1.0f && std::floor(std::fma(last, scale[a], bias[a])) <= float(i);
 			}
 		}
+		if (holds) return level;
 	}
-	return grid;
+	return 0;
+}
+
+void gridOf(const FlatWorld& flat, uint32_t level, uint32_t fine, std::vector<uint32_t>& grid, std::vector<uint32_t>& bricks) {
+	const auto entryOf = [&](int32_t node, uint32_t at) {
+		if (node >= 0) return uint32_t(node);
+		const uint32_t leaf = uint32_t(~node);
+		return kEntryLeaf | (flat.leaves[leaf].shape == ShapeEmpty ? kEntryEmpty : 0u) | at << kEntryLevelShift | leaf;
+	};
+	// the entries `wide` levels below a node, each node that ends above them
+	// over all of its cells; what is still inner goes on as a brick
+	struct Part {
+		int32_t node;
+		uint32_t level, x, y, z;
+	};
+	struct Inner {
+		int32_t node;
+		uint32_t level;
+		size_t entry;
+	};
+	std::vector<Part> parts;
+	std::vector<Inner> inner;
+	const auto fill = [&](std::vector<uint32_t>& to, size_t base, int32_t node, uint32_t from, uint32_t down, uint32_t row) {
+		const uint32_t end = from + down;
+		parts.push_back({ node, from, 0, 0, 0 });
+		while (!parts.empty()) {
+			const Part p = parts.back();
+			parts.pop_back();
+			if (p.level < end && p.node >= 0) {
+				for (uint32_t o = 0; o < 8; ++o) parts.push_back({ flat.nodes[size_t(p.node) + o], p.level + 1, p.x * 2 + (o & 1u), p.y * 2 + (o >> 1 & 1u), p.z * 2 + (o >> 2) });
+				continue;
+			}
+			const uint32_t wide  = 1u << (end - p.level);
+			const uint32_t entry = entryOf(p.node, p.level);
+			for (uint32_t z = p.z * wide; z < (p.z + 1) * wide; ++z) {
+				for (uint32_t y = p.y * wide; y < (p.y + 1) * wide; ++y) {
+					std::fill_n(to.begin() + std::ptrdiff_t(base + (size_t(z) * row + y) * row + size_t(p.x) * wide), wide, entry);
+				}
+			}
+			if (p.node >= 0 && end < fine) inner.push_back({ p.node, end, base + (size_t(p.z) * row + p.y) * row + p.x });
+		}
+	};
+	grid.assign(size_t(1) << (3 * level), 0);
+	bricks.clear();
+	fill(grid, 0, flat.nodes[0], 0, level, 1u << level);
+	bool inGrid = true;
+	while (!inner.empty()) {
+		std::vector<Inner> here;
+		here.swap(inner);
+		for (const Inner& n : here) {
+			const size_t base                  = bricks.size();
+			(inGrid ? grid : bricks)[n.entry] = uint32_t(base / kBrick);
+			bricks.resize(base + kBrick, 0);
+			fill(bricks, base, n.node, n.level, std::min(2u, fine - n.level), 4);
+		}
+		inGrid = false;
+	}
 }
 
 } // namespace kdn

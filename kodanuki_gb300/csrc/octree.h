@@ -53,10 +53,15 @@ struct FlatWorld {
 // Returns an empty string, or what went wrong.
 std::string buildOctree(const std::vector<ProgPtr>& objects, const double lower[3], const double size[3], const BuildOptions& options, Octree& tree);
 std::string flattenOctree(const Octree& tree, FlatWorld& flat);
-// The grid of `level` over a flattened octree (world.h GridCell).
-std::vector<GridCell> gridOf(const FlatWorld& flat, uint32_t level);
-// The walls of that grid per axis (3 x (2^level + 1)): the descent's
-// midpoints in FP32 over [lower, lower + size].
-std::vector<float> gridWallsOf(const float lower[3], const float size[3], uint32_t level);
+// The grid of `level` over a flattened octree and the bricks from it down to
+// `fine` (world.h kEntryLeaf).
+void gridOf(const FlatWorld& flat, uint32_t level, uint32_t fine, std::vector<uint32_t>& grid, std::vector<uint32_t>& bricks);
+// The walls of `level` per axis (3 x (2^level + 1)): the descent's midpoints
+// in FP32 over [lower, lower + size].
+std::vector<float> wallsOf(const float lower[3], const float size[3], uint32_t level);
+// How a point's place among them is estimated, and the finest level (most at
+// most) at which the estimate holds (world.h kMostFine).
+void placeScale(const float lower[3], const float size[3], uint32_t level, float scale[3], float bias[3]);
+uint32_t fineLevelOf(const float lower[3], const float size[3], uint32_t most);
 
 } // namespace kdn

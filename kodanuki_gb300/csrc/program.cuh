@@ -126,83 +126,80 @@ KDN_HD float addAlone(float a, float b) {
 #endif
 }
 
-// world.h FormAxis: a coordinate's distance to a slab.
-KDN_HD float axisValue(float p, uint32_t side, const MarchParams& q) {
-	float u = addAlone(p, -q.v[0]);
+// A coordinate's distance to a slab: side of p - c, then - h, + r (and - e).
+KDN_HD float slabValue(float p, uint32_t side, float c, float h, float r) {
+	float u = addAlone(p, -c);
 	u       = side == SideAbs ? fabsf(u) : u;
 	u       = side == SideNegative ? 0.0f - u : u;
-	return addAlone(addAlone(addAlone(u, -q.v[1]), q.v[2]), -q.v[3]);
+	return addAlone(addAlone(u, -h), r);
 }
+KDN_HD float axisValue(float p, uint32_t side, const MarchParams& q) { return addAlone(slabValue(p, side, q.v[0], q.v[1], q.v[2]), -q.v[3]); }
 
-// world.h FormSphere.
+// A point's distance to a sphere: centre and radius.
 KDN_HD float sphereValue(float px, float py, float pz, const MarchParams& q) {
 	const float x = addAlone(px, -q.v[0]), y = addAlone(py, -q.v[1]), z = addAlone(pz, -q.v[2]);
 	return addAlone(marchSqrt(fmaf(z, z, fmaf(x, x, mulAlone(y, y)))), -q.v[3]);
 }
 
-// world.h FormNorm over the values of its slots.
-KDN_HD float normValue(float a, float b, float c, float m, uint32_t flags, float e) {
-	const float p = flags & NormPositive0 ? fmaxf(a, 0.0f) : a;
-	const float q = flags & NormPositive1 ? fmaxf(b, 0.0f) : b;
-	const float r = flags & NormPositive2 ? fmaxf(c, 0.0f) : c;
+// The sum of squares of a root's terms (world.h SumFlag); a term left out
+// adds an exact zero.
+KDN_HD float squaresOf(float a, float b, float c, uint32_t flags) {
+	const float p = flags & SumHas0 ? (flags & SumPositive0 ? fmaxf(a, 0.0f) : a) : 0.0f;
+	const float q = flags & SumHas1 ? (flags & SumPositive1 ? fmaxf(b, 0.0f) : b) : 0.0f;
+	const float r = flags & SumHas2 ? (flags & SumPositive2 ? fmaxf(c, 0.0f) : c) : 0.0f;
 	float sum     = mulAlone(p, p);
-	sum           = flags & NormFused1 ? fmaf(q, q, sum) : addAlone(mulAlone(q, q), sum);
-	const float s = flags & NormFused2 ? fmaf(r, r, sum) : addAlone(mulAlone(r, r), sum);
-	float f       = marchSqrt(flags & NormThree ? s : sum);
-	if (flags & NormInside) {
-		if (flags & NormInsideMax) {
-			m = flags & NormThree ? (b < c ? c : b) : b;
-			m = a < m ? m : a;
-		}
-		f = addAlone(f, 0.0f < m ? 0.0f : m);
-	}
-	return addAlone(f, -e);
+	sum           = flags & SumFused1 ? fmaf(q, q, sum) : addAlone(mulAlone(q, q), sum);
+	return flags & SumFused2 ? fmaf(r, r, sum) : addAlone(mulAlone(r, r), sum);
 }
 
-// One step of the march form (world.h MarchStep) and, of a fused step, its
-// parameters: r = post(form, w), with the post operations worked out
-// together and the step's picked, so the lanes of a warp on different posts
-// do not split; a rare step runs the reference operation.  Writes the result
-// to its slot.
-KDN_HD void marchStep(const MarchStep& s, const MarchParams& q, float* slots, uint32_t stride) {
-	float r;
-	if (s.op >= kMarchRare) {
-		slots[SlotImm * stride] = s.value;
-		const float a = slots[s.a * stride], b = slots[s.b * stride], c = slots[s.c * stride];
-		const float p[3] = { slots[SlotX * stride], slots[SlotY * stride], slots[SlotZ * stride] };
-		r                = stepValue(uint8_t(s.op - kMarchRare), a, b, c, s.value, p);
-	} else {
-		const uint32_t form = s.op & kMarchFormMask, post = s.op & kMarchPostMask;
-		float f;
-		if (form == FormAxis) {
-			f = axisValue(slots[s.a * stride], s.flags, q);
-		} else if (form == FormSphere) {
-			f = sphereValue(slots[SlotX * stride], slots[SlotY * stride], slots[SlotZ * stride], q);
-		} else if (form == FormNorm) {
-			f = normValue(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride], slots[s.m * stride], s.flags, q.v[0]);
-		} else {
-			slots[SlotImm * stride] = s.value;
-			f                       = fmaf(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride]);
-		}
-		r = f;
-		if (post != PostNone) {
-			slots[SlotImm * stride] = s.value;
-			const float w = slots[s.w * stride];
-			const float p = fmaxf(f, 0.0f);
-			// the smooth minimum of radius r = value: min - max(r - |f - w|, 0)^2 * 0.25 / r
-			const float m = fmaxf(s.value - fabsf(f - w), 0.0f);
-			r             = post == PostSqrt ? marchSqrt(f) : r;
-			r             = post == PostAbs ? fabsf(f) : r;
-			r             = post == PostPosSq ? p * p : r;
-			r             = post == PostMin ? (w < f ? w : f) : r;
-			r             = post == PostMax ? (f < w ? w : f) : r;
-			r             = post == PostSminK ? fminf(f, w) - m * m * s.quarter : r;
-		}
+KDN_HD float greaterOf(float f, float w) { return f < w ? w : f; } // PostMax
+KDN_HD float belowZero(float m) { return 0.0f < m ? 0.0f : m; }    // PostMin with 0
+
+// world.h FormPrimitive at a point.
+KDN_HD float primitiveValue(const MarchStep& s, const MarchParams& c, const MarchParams& h, float px, float py, float pz) {
+	const uint32_t terms[3] = { s.a, s.b, s.c };
+	float u[3];
+	for (int k = 0; k < 3; ++k) {
+		const uint32_t axis = terms[k] & 3u;
+		u[k]                = slabValue(axis == 0 ? px : axis == 1 ? py : pz, terms[k] >> kTermSideShift, c.v[k], h.v[k], h.v[3]);
 	}
-	slots[s.dst * stride] = r;
+	float f = marchSqrt(squaresOf(u[0], u[1], u[2], s.flags));
+	if (s.m & PrimSingle) f = greaterOf(s.flags & SumHas0 ? u[0] : s.flags & SumHas1 ? u[1] : u[2], 0.0f);
+	if (s.m & PrimPlain) f = u[0];
+	const float inside = belowZero(greaterOf(u[0], s.m & PrimThird ? greaterOf(u[1], u[2]) : u[1]));
+	f                  = s.m & PrimInside ? addAlone(f, inside) : f;
+	return addAlone(f, -c.v[3]);
 }
 
-// The parameters of a fused step, in the unit after it.
+// The post operation of a step's value f, worked out together and the step's
+// picked, so the lanes of a warp on different posts do not split.
+KDN_HD float posted(uint32_t post, float f, float w, float value, float quarter) {
+	const float p = fmaxf(f, 0.0f);
+	// the smooth minimum of radius r = value: min - max(r - |f - w|, 0)^2 * 0.25 / r
+	const float m = fmaxf(value - fabsf(f - w), 0.0f);
+	float r       = f;
+	r             = post == PostSqrt ? marchSqrt(f) : r;
+	r             = post == PostAbs ? fabsf(f) : r;
+	r             = post == PostPosSq ? p * p : r;
+	r             = post == PostMin ? (w < f ? w : f) : r;
+	r             = post == PostMax ? (f < w ? w : f) : r;
+	r             = post == PostSminK ? fminf(f, w) - m * m * quarter : r;
+	return r;
+}
+
+// A rare step's reference operation; out of line on the device, where its
+// sines and powers would otherwise be laid into every march loop.
+#ifdef __CUDA_ARCH__
+__device__ __noinline__
+#else
+inline
+#endif
+float rareValue(uint8_t op, float a, float b, float c, float value, float3 at) {
+	const float p[3] = { at.x, at.y, at.z };
+	return stepValue(op, a, b, c, value, p);
+}
+
+// The parameters of a fused step, a unit.
 KDN_HD MarchParams paramsAt(const MarchStep* unit) {
 #ifdef __CUDA_ARCH__
 	const float4 v = *reinterpret_cast<const float4*>(unit);
@@ -214,20 +211,70 @@ KDN_HD MarchParams paramsAt(const MarchStep* unit) {
 #endif
 }
 
-// Whether a step is a fused one.
-KDN_HD bool fusedStep(const MarchStep& s) { return s.op < kMarchRare && (s.op & kMarchFormMask) != FormFma; }
+// One step of the march form (world.h MarchStep) at a point but a primitive,
+// over a thread's slots: r = post(form, w); a rare step runs the reference
+// operation.  Writes the result to its slot and returns it.
+KDN_HD float marchStep(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride) {
+	slots[SlotImm * stride] = s.value;
+	float r;
+	if (s.op >= kMarchRare) {
+		const float a = slots[s.a * stride], b = slots[s.b * stride], c = slots[s.c * stride];
+		r = rareValue(uint8_t(s.op - kMarchRare), a, b, c, s.value, make_float3(slots[SlotX * stride], slots[SlotY * stride], slots[SlotZ * stride]));
+	} else {
+		const uint32_t form = s.op & kMarchFormMask, post = s.op & kMarchPostMask;
+		if (form == FormNorm) {
+			r = marchSqrt(squaresOf(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride], s.flags));
+			if (s.m != kNoInside) r = addAlone(r, belowZero(slots[s.m * stride]));
+			r = addAlone(r, -paramsAt(unit).v[0]);
+		} else if (form == FormRepeat) {
+			const float x = slots[s.a * stride];
+			r             = addAlone(x, -mulAlone(s.value, floorf(addAlone(x / s.value, s.quarter))));
+		} else {
+			r = fmaf(slots[s.a * stride], slots[s.b * stride], slots[s.c * stride]);
+		}
+		if (post != PostNone) r = posted(post, r, slots[s.w * stride], s.value, s.quarter);
+	}
+	slots[s.dst * stride] = r;
+	return r;
+}
+
+// The units of a step.
+KDN_HD uint32_t unitsOf(const MarchStep& s) {
+	const uint32_t form = s.op & kMarchFormMask;
+	return s.op >= kMarchRare || form == FormFma || form == FormRepeat ? 1u : form == FormPrimitive && s.m & PrimSized ? 3u : 2u;
+}
+KDN_HD bool primitiveStep(const MarchStep& s) { return s.op < kMarchRare && (s.op & kMarchFormMask) == FormPrimitive; }
+
+// A primitive step at a point; last is the step before's result.
+KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride, float px, float py, float pz, float last) {
+	const MarchParams c = paramsAt(unit);
+	MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
+	if (s.m & PrimSized) h = paramsAt(unit + 1);
+	float r             = primitiveValue(s, c, h, px, py, pz);
+	const uint32_t post = s.op & kMarchPostMask;
+	if (post != PostNone) {
+		float w = last;
+		if (!(s.m & PrimPrevious)) w = s.w == SlotImm ? s.value : slots[s.w * stride];
+		r = posted(post, r, w, s.value, s.quarter);
+	}
+	if (s.m & PrimStored) slots[s.dst * stride] = r;
+	return r;
+}
 
 // One program at one point; slots is this thread's column base (stride
-// blockDim.x), with the constants set.  Returns the program's value.
-KDN_HD float evalSlots(const MarchStep* __restrict__ code, uint32_t count, uint32_t resultSlot, float* slots, uint32_t stride, const float p[3]) {
+// blockDim.x), with the constants set.  Returns the program's value, which
+// its last step makes.
+KDN_HD float evalSlots(const MarchStep* __restrict__ code, uint32_t count, float* slots, uint32_t stride, const float p[3]) {
 	setPoint(slots, stride, p);
-	for (uint32_t i = 0; i < count; ++i) {
+	float last = 0.0f;
+#pragma unroll 1
+	for (uint32_t i = 0; i < count;) {
 		const MarchStep s = code[i];
-		MarchParams q {};
-		if (fusedStep(s)) q = paramsAt(code + ++i);
-		marchStep(s, q, slots, stride);
+		if (primitiveStep(s)) last = primitiveStepValue(s, code + i + 1, slots, stride, p[0], p[1], p[2], last);
+		else last = marchStep(s, code + i + 1, slots, stride);
+		i += unitsOf(s);
 	}
-	return slots[resultSlot * stride];
+	return last;
 }
 
 struct DualF {

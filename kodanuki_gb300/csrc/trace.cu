@@ -19,13 +19,14 @@ namespace kdn {
 namespace {
 
 constexpr int kTraceBlock = 128;
-// program steps a thread runs a turn of the step machine before the warp
-// looks again for threads that need a new ray or a new cell (8 measured
-// faster than 4 on config 2: fewer turns of overhead a program, whose march
-// form is ~6 steps on average)
-constexpr uint32_t kStepsPerTurn = 8;
-// empty cells a thread passes a turn before the warp moves on
-constexpr uint32_t kCellsPerTurn = 1;
+// A thread's register slots are a column of shared memory, one float a slot.
+constexpr uint32_t kStride = kTraceBlock;
+// cells a turn takes a ray through while they are empty, march steps inside a
+// shaped cell (world.h LeafShape) and program steps, before the warp looks again at what most of its
+// rays wait for
+constexpr uint32_t kCellsPerTurn = 3;
+constexpr uint32_t kMovesPerTurn = 8;
+constexpr uint32_t kStepsPerTurn = 4;
 
 __device__ __forceinline__ float slopeOf(float part) {
 	const float tiny = 1e-12f;
@@ -39,98 +40,91 @@ __device__ __forceinline__ float tolerance(const float p[3]) {
 
 __device__ __forceinline__ float nudge(float t) { return fmaxf(1e-5f, fabsf(t) * 2e-6f); }
 
-__device__ __forceinline__ float cellExitBy(const float o[3], const float inv[3], const Located& l) {
-	float up = 3.0e38f;
-	for (int a = 0; a < 3; ++a) {
-		const float x = (l.lo[a] - o[a]) * inv[a];
-		const float y = (l.hi[a] - o[a]) * inv[a];
-		up            = fminf(up, fmaxf(x, y));
-	}
-	return up;
+// Where a ray leaves the cell it is in: its walls ahead, one an axis.  A march
+// only goes forward and p = o + d t rounds monotonically, so a ray in a cell
+// leaves it by these walls alone and the three behind it are never looked at.
+// They are kept as the ray sees them, with the sign of its direction taken off
+// both sides: up an axis it is in the cell while p < upper, down an axis while
+// p >= lower, which is -p < the next number above -lower.
+__device__ __forceinline__ float forward(float p, float d) { return __uint_as_float(__float_as_uint(p) ^ (__float_as_uint(d) & 0x80000000u)); }
+
+__device__ __forceinline__ bool inside(const float wall[3], const float p[3], const float d[3]) {
+	return forward(p[0], d[0]) < wall[0] && forward(p[1], d[1]) < wall[1] && forward(p[2], d[2]) < wall[2];
 }
 
-__device__ __forceinline__ float cellExit(const float o[3], const float d[3], const Located& l) {
-	float up = 3.0e38f;
-	for (int a = 0; a < 3; ++a) {
-		const float inv = slopeOf(d[a]);
-		const float x   = (l.lo[a] - o[a]) * inv;
-		const float y   = (l.hi[a] - o[a]) * inv;
-		up              = fminf(up, fmaxf(x, y));
-	}
-	return up;
-}
-
-struct Field {
-	float least;   // least program value
-	float nearest; // least magnitude
-	uint32_t index;  // which kept program is least
-	uint32_t count;  // kept programs
-	uint32_t first;  // first GpuProgram of the leaf
-	bool empty;
+// A cell ahead of a ray: its leaf, its walls, and the parameter the ray
+// reaches them at (of an axis's two walls (w - o) * inv is never less at the
+// one ahead).
+struct Ahead {
+	uint32_t leaf;
+	float wall[3];
 	float exit;
 };
 
-// Whether a point is in a located cell: the half-open box the descent gives
-// it (a coordinate equal to a midpoint goes to the upper half), so a point
-// found here is the point the descent would find there.
-__device__ __forceinline__ bool within(const Located& l, const float p[3]) {
-	return l.leaf != kNoLeaf && p[0] >= l.lo[0] && p[0] < l.hi[0] && p[1] >= l.lo[1] && p[1] < l.hi[1] && p[2] >= l.lo[2] && p[2] < l.hi[2];
+__device__ __forceinline__ void walledBy(Ahead& c, const float at[3], const float o[3], const float d[3], const float inv[3]) {
+	c.exit = 3.0e38f;
+	for (int a = 0; a < 3; ++a) {
+		const float back  = 0.0f - at[a]; // +0 for a wall at 0
+		const int32_t bit = __float_as_int(back);
+		c.wall[a]         = __float_as_int(d[a]) < 0 ? __int_as_float(bit < 0 ? bit - 1 : bit + 1) : at[a];
+		c.exit            = fminf(c.exit, (at[a] - o[a]) * inv[a]);
+	}
 }
 
-// The field at t from the kept programs of the cell the point lies in.  The
-// cell of the previous step is kept in `cell`: a ray takes several steps in
-// one cell, and only a point that has left it descends the octree again.
-__device__ __forceinline__ Field fieldAt(const DeviceWorld& w, const float o[3], const float d[3], float t, float* slots, uint32_t stride, uint32_t& steps, Located& cell) {
-	Field f;
-	const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-	if (!within(cell, p)) cell = locate(w, p);
-	const Located& l   = cell;
-	const GpuLeaf leaf = w.leaves[l.leaf];
-	f.first  = leaf.first;
-	f.count  = leaf.count;
-	f.empty  = leaf.occupancy == Empty || leaf.count == 0;
-	f.least  = 3.0e38f;
-	f.nearest = 3.0e38f;
-	f.index  = 0;
-	// A cell keeps only the objects whose surface may pass through it
-	// (cut.cpp:442 deciding), so past its walls its field is no distance
-	// bound: a step stops where the ray leaves the cell.
-	f.exit   = cellExit(o, d, l);
-	if (f.empty) return f;
-	for (uint32_t k = 0; k < leaf.count; ++k) {
-		const GpuProgram g = w.programs[leaf.first + k];
-		const float v      = evalSlots(w.march + g.march, g.marchCount, g.marchSlot, slots, stride, p);
-		steps += g.marchCount;
+// A leaf below the finest tabled level: the descent goes on by midpoints.
+__device__ __noinline__ Ahead deepCell(const DeviceWorld& w, float3 point, int32_t node, int3 at, float3 origin, float3 along, float3 inverse) {
+	const float p[3] = { point.x, point.y, point.z }, o[3] = { origin.x, origin.y, origin.z };
+	const float d[3] = { along.x, along.y, along.z }, inv[3] = { inverse.x, inverse.y, inverse.z };
+	const int place[3] = { at.x, at.y, at.z };
+	float lo[3], hi[3];
+	for (int a = 0; a < 3; ++a) {
+		const float* walls = w.walls + a * ((1 << w.fineLevel) + 1) + place[a];
+		lo[a]              = walls[0];
+		hi[a]              = walls[1];
+	}
+	Ahead c;
+	c.leaf = uint32_t(~descend(w, p, node, lo, hi));
+	for (int a = 0; a < 3; ++a) lo[a] = __float_as_int(d[a]) < 0 ? lo[a] : hi[a];
+	walledBy(c, lo, o, d, inv);
+	return c;
+}
+
+struct Field {
+	float least;    // least program value
+	uint32_t index; // which kept program is least
+	uint32_t count; // kept programs
+	uint32_t first; // first GpuProgram of the leaf
+};
+
+// The field at p from the kept programs of its cell; no programs in an empty one.
+__device__ __forceinline__ Field fieldAt(const DeviceWorld& w, const float p[3], float* slots, uint32_t& steps) {
+	const GpuLeaf leaf = w.leaves[locate(w, p)];
+	Field f { 3.0e38f, 0, leaf.shape == ShapeEmpty ? 0u : leaf.count, leaf.first };
+	for (uint32_t k = 0; k < f.count; ++k) {
+		const GpuProgram g = w.programs[f.first + k];
+		const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
+		steps += g.marchSteps;
 		if (v < f.least) {
 			f.least = v;
 			f.index = k;
 		}
-		f.nearest = fminf(f.nearest, fabsf(v));
 	}
 	return f;
 }
 
-// The least value at t, and the index of the kept program that is least a
+// The least value at p, and the index of the kept program that is least a
 // little further along among those tied with it (sphere_trace.cpp:96).
-__device__ __forceinline__ uint32_t winnerAt(const DeviceWorld& w, const float o[3], const float d[3], float t, const Field& f, float* slots, uint32_t stride) {
-	const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+__device__ __noinline__ uint32_t winnerAt(const DeviceWorld& w, float3 at, float3 along, const Field f, float* slots) {
+	const float p[3] = { at.x, at.y, at.z };
 	const float big  = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
 	const float band = 2e-6f * (1.0f + big);
-	const float q[3] = { p[0] + d[0] * 2e-5f, p[1] + d[1] * 2e-5f, p[2] + d[2] * 2e-5f };
+	const float q[3] = { p[0] + along.x * 2e-5f, p[1] + along.y * 2e-5f, p[2] + along.z * 2e-5f };
 	uint32_t winner  = f.index;
 	float onWinner   = 3.0e38f;
-	bool tied        = false;
-	float values[kMaxLeafProgs];
-	for (uint32_t k = 0; k < f.count && k < kMaxLeafProgs; ++k) {
+	for (uint32_t k = 0; k < f.count; ++k) {
 		const GpuProgram g = w.programs[f.first + k];
-		values[k]          = evalSlots(w.march + g.march, g.marchCount, g.marchSlot, slots, stride, p);
-		tied               = tied || (k != f.index && values[k] - f.least <= band);
-	}
-	if (!tied) return winner;
-	for (uint32_t k = 0; k < f.count && k < kMaxLeafProgs; ++k) {
-		if (!(values[k] - f.least <= band)) continue;
-		const GpuProgram g = w.programs[f.first + k];
-		const float on     = evalSlots(w.march + g.march, g.marchCount, g.marchSlot, slots, stride, q);
+		if (!(evalSlots(w.march + g.march, g.marchCount, slots, kStride, p) - f.least <= band)) continue;
+		const float on = evalSlots(w.march + g.march, g.marchCount, slots, kStride, q);
 		if (on < onWinner) {
 			onWinner = on;
 			winner   = k;
@@ -139,43 +133,38 @@ __device__ __forceinline__ uint32_t winnerAt(const DeviceWorld& w, const float o
 	return winner;
 }
 
-// sphereFromInside at a point within the tolerance of the nearest surface:
-// read the field a little past it.  kind 0: go on past (t += inset); 1: the
-// ray leaves its solid here (winner among the cell's programs); 2: it meets
-// a solid of another material (the program past the point).
+// sphereFromInside at a point p within the tolerance of the nearest surface:
+// read the field a little past it, at q.  kind 0: go on past (t += inset); 1:
+// the ray leaves its solid here (winner among the cell's programs); 2: it
+// meets a solid of another material (the program past the point).
 struct InsideStop {
-	uint32_t kind, first, index;
+	uint32_t kind, first, index, steps;
 };
 
-__device__ __forceinline__ InsideStop insideStop(const DeviceWorld& w, const uint32_t* objectMaterial, uint32_t medium, const float o[3], const float d[3], float t,
-                                             float inset, const Field& f, const Located& cell, float* slots, uint32_t stride, uint32_t& steps) {
-	Located beyond   = cell;
-	const Field past = fieldAt(w, o, d, t + inset, slots, stride, steps, beyond);
-	if (past.empty || past.least > 0.0f) return InsideStop { 1, f.first, winnerAt(w, o, d, t, f, slots, stride) };
+__device__ __noinline__ InsideStop insideStop(const DeviceWorld& w, const uint32_t* objectMaterial, uint32_t medium, float3 p, float3 q, float3 along, const Field f, float* slots) {
+	const float beyond[3] = { q.x, q.y, q.z };
+	uint32_t steps        = 0;
+	const Field past      = fieldAt(w, beyond, slots, steps);
+	if (past.count == 0 || past.least > 0.0f) return InsideStop { 1, f.first, winnerAt(w, p, along, f, slots), steps };
 	const GpuProgram g = w.programs[past.first + past.index];
 	// a solid of another material than the one the ray is in: stop there
-	if (objectMaterial != nullptr && objectMaterial[g.object] != medium) return InsideStop { 2, past.first, past.index };
-	return InsideStop { 0, 0, 0 };
+	if (objectMaterial != nullptr && objectMaterial[g.object] != medium) return InsideStop { 2, past.first, past.index, steps };
+	return InsideStop { 0, 0, 0, steps };
 }
 
-// The march as a step machine.  Each thread holds one ray at a time and
-// every turn of the loop runs one program step for every thread that is
-// evaluating, so threads whose cells hold programs of different lengths, or
-// whose rays take different numbers of march steps, stay busy: a thread that
-// finishes a program moves on to the next program of its cell, a thread that
-// finishes a march step locates its next cell, and a thread whose ray ends
-// takes the next ray of the launch (one atomic a warp).
-enum LaneMode : uint32_t { Fetch = 0, Locating = 1, Evaluating = 2, Finished = 3 };
+// The march as a step machine.  Each thread holds one ray at a time.  A ray
+// waits to be located, or to step in a cell whose field its leaf record holds
+// (empty, or a single slab or sphere: a few operations in registers), or for
+// the programs of its cell, a few of their steps at a time; every turn the
+// warp does what most of its rays wait for.  A ray that ends takes the next
+// ray of the launch (one atomic a warp).
+enum LaneMode : uint32_t { Fetch = 0, Locating = 1, Stepping = 2, Evaluating = 3, Finished = 4 };
 
-// Seven blocks an SM is what 72 registers a thread allow; saying so lets
-// ptxas keep the step machine's state in registers (it spills 8 bytes with
-// the hint, 44 without; 46.1 against 45.3 Msamples/s on config 2).
-__global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
+__global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_constant__ TraceArgs args) {
 	extern __shared__ float slotMemory[];
-	const DeviceWorld& w  = args.world;
-	const uint32_t stride = blockDim.x;
-	float* slots          = slotMemory + threadIdx.x;
-	setConstants(slots, stride);
+	const DeviceWorld& w = args.world;
+	float* slots         = slotMemory + threadIdx.x;
+	setConstants(slots, kStride);
 	// capped rays in the low 16 bits, carried ones in the high: one register
 	uint32_t marchSteps = 0, programSteps = 0, traced = 0, cappedCarried = 0, longest = 0;
 	// the steps a ray may take in this launch: a launch's budget, or the cap
@@ -193,22 +182,22 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 	uint32_t ray  = 0;
 	float o[3], d[3], inv[3];
 	float t = 0.0f, up = 0.0f;
-	bool inside      = false;
-	uint32_t medium  = kNoLeaf;
-	uint32_t step    = 0;
+	bool within   = false; // the ray started inside a solid
+	uint32_t step = 0;
 	// where the ray's march stops in this launch: the cap, or sooner its budget
 	uint32_t stepLimit = 0;
-	Located cell;
-	cell.leaf = kNoLeaf;
-	float exitT = 0.0f;
-	// the cell being evaluated: its run of kept programs and the one in hand
-	uint32_t first = 0, count = 0, k = 0;
-	const MarchStep* code = nullptr;
+	// the ray's cell, its shape, and what a step in it adds to the program step count
+	uint32_t shape = 0, cost = 0;
+	Ahead cell { kNoLeaf, { 0.0f, 0.0f, 0.0f }, 0.0f };
+	// the field of a slab or a sphere; in a cell of programs, what the ones
+	// evaluated so far came to: v[0] the least value, v[1] the second least
+	// (from inside a solid, the least magnitude)
+	MarchParams field { { 0.0f, 0.0f, 0.0f, 0.0f } };
+	// the program in hand: its code from pc to end, its last step's value, and
+	// which it is, of how many, and which was least (a byte each)
+	uint32_t pc = 0, end = 0, order = 0;
+	float last = 0.0f;
 	MarchStep next {};
-	uint32_t pc = 0, length = 0, resultSlot = 0;
-	float p[3]  = { 0.0f, 0.0f, 0.0f };
-	float least = 0.0f, second = 0.0f, nearest = 0.0f;
-	uint32_t index = 0;
 	// a ray ends: its state, the step counts, and the next ray
 	auto done = [&](HitState h) {
 		args.states[ray] = h;
@@ -216,6 +205,15 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 		longest = max(longest, h.steps);
 		cappedCarried += h.kind == kCarried ? 0x10000u : (h.steps >= args.maxSteps ? 1u : 0u);
 		mode = Fetch;
+	};
+	// past the cap or the region: a miss, which keeps where its march stopped
+	// (a held path resumes it); out of this launch's budget before either:
+	// carried, the march's whole state being (t, step)
+	auto over = [&]() {
+		if (step < stepLimit && t <= up) return false;
+		const bool carried = step < args.maxSteps && t <= up;
+		done(HitState { carried ? kCarried : 0u, t, kNoLeaf, 0, step });
+		return true;
 	};
 
 	for (;;) {
@@ -234,6 +232,7 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 				} else {
 					if (ray >= n1) ray = args.second + (ray - n1);
 					const kdn_ray r = args.rays[ray];
+					within          = r.inside != 0;
 					for (int a = 0; a < 3; ++a) {
 						o[a]   = r.origin[a];
 						d[a]   = r.direction[a];
@@ -247,10 +246,8 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 						lo            = fmaxf(lo, fminf(x, y));
 						up            = fminf(up, fmaxf(x, y));
 					}
-					t         = lo;
-					inside    = r.inside != 0;
-					medium    = r.within;
-					step      = 0;
+					t    = lo;
+					step = 0;
 					// a carried ray goes on where its march stood
 					if (args.carry != nullptr && (r.pad_[0] & kRayResumes)) {
 						const uint2 c = args.carry[ray];
@@ -261,119 +258,187 @@ __global__ void __launch_bounds__(kTraceBlock, 7) traceKernel(TraceArgs args) {
 					}
 					stepLimit = min(args.maxSteps, step + allowance);
 					marchSteps -= step;
-					cell.leaf = kNoLeaf;
-					if (up < lo) {
-						done(HitState { 0, t, kNoLeaf, 0, step });
-					} else {
-						mode = Locating;
-					}
+					if (up < lo) done(HitState { 0, t, kNoLeaf, 0, step });
+					else if (!over()) mode = Locating;
 				}
 			}
 		}
-		if (__all_sync(0xFFFFFFFFu, mode == Finished)) break;
-
-		// find the cell of the point, skipping empty cells, and start its first program
-		if (mode == Locating) {
-			for (uint32_t skipped = 0;;) {
-				// past the cap or the region: a miss, which keeps where its march
-				// stopped (a held path resumes it); out of this launch's budget
-				// before either: carried, the march's whole state being (t, step)
-				if (!(step < stepLimit && t <= up)) {
-					const bool carried = step < args.maxSteps && t <= up;
-					done(HitState { carried ? kCarried : 0u, t, kNoLeaf, 0, step });
-					break;
+		const int locating   = __popc(__ballot_sync(0xFFFFFFFFu, mode == Locating));
+		const int stepping   = __popc(__ballot_sync(0xFFFFFFFFu, mode == Stepping));
+		const int evaluating = __popc(__ballot_sync(0xFFFFFFFFu, mode == Evaluating));
+		if (locating + stepping + evaluating == 0) {
+			if (__all_sync(0xFFFFFFFFu, mode == Finished)) break;
+			continue;
+		}
+		// a march step whose value is worked out: the least of the cell's
+		// programs, the second least (from inside, the least magnitude), the least's index
+		bool whole     = false;
+		float least    = 0.0f, second = 0.0f;
+		uint32_t index = 0;
+		bool start     = false; // a ray starts on its cell's programs
+		if (evaluating > locating && evaluating > stepping) {
+			if (mode == Evaluating) {
+				// a few program steps; each step's code is loaded a step ahead
+				const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+#pragma unroll 1
+				for (uint32_t u = 0; u < kStepsPerTurn; ++u) {
+					const MarchStep s     = next;
+					const MarchStep* unit = w.march + pc + 1;
+					pc += unitsOf(s);
+					if (pc < end) next = w.march[pc];
+					if (primitiveStep(s)) {
+						last = primitiveStepValue(s, unit, slots, kStride, p[0], p[1], p[2], last);
+					} else {
+						setPoint(slots, kStride, p);
+						last = marchStep(s, unit, slots, kStride);
+					}
+					if (pc == end) break;
 				}
-				for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
-				if (!within(cell, p)) cell = locate(w, p);
+				if (pc == end) {
+					const float v = last;
+					programSteps += cost;
+					uint32_t k        = order >> 8 & 0xFFu;
+					const bool lesser = v < field.v[0];
+					field.v[1]        = within ? fminf(field.v[1], fabsf(v)) : lesser ? field.v[0] : fminf(field.v[1], v);
+					field.v[0]        = lesser ? v : field.v[0];
+					if (lesser) order = (order & 0x0000FFFFu) | k << 16;
+					if (++k < (order & 0xFFu)) {
+						const GpuProgram g = w.programs[w.leaves[cell.leaf].first + k];
+						pc    = g.march;
+						end   = g.march + g.marchCount;
+						order = (order & 0x00FF00FFu) | k << 8;
+						cost  = g.marchSteps;
+						next  = w.march[pc];
+					} else {
+						least  = field.v[0];
+						second = field.v[1];
+						index  = order >> 16;
+						whole  = true;
+					}
+				}
+			}
+		} else {
+			if (mode == Locating && locating >= stepping) {
+				// the cell of the point; an empty one is left at once, for the next
+#pragma unroll 1
+				for (uint32_t u = 0; u < kCellsPerTurn; ++u) {
+					const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+					int place[3];
+					placeOf(w, p, place);
+					const uint32_t entry = entryAt(w, place);
+					bool empty           = entry & kEntryEmpty;
+					if (entry & kEntryLeaf) {
+						const uint32_t wide = w.fineLevel - (entry >> kEntryLevelShift & 15u), row = (1u << w.fineLevel) + 1u;
+						float at[3];
+						for (int a = 0; a < 3; ++a) at[a] = __ldg(w.walls + a * row + ((uint32_t(place[a]) >> wide) + (__float_as_int(d[a]) < 0 ? 0u : 1u) << wide));
+						walledBy(cell, at, o, d, inv);
+						cell.leaf = entry & kEntryIndex;
+					} else {
+						cell  = deepCell(w, make_float3(p[0], p[1], p[2]), int32_t(entry), make_int3(place[0], place[1], place[2]), make_float3(o[0], o[1], o[2]), make_float3(d[0], d[1], d[2]), make_float3(inv[0], inv[1], inv[2]));
+						empty = w.leaves[cell.leaf].shape == ShapeEmpty;
+					}
+					if (!empty) {
+						const GpuLeaf leaf = w.leaves[cell.leaf];
+						shape              = leaf.shape;
+						cost               = leaf.marchSteps;
+						for (int a = 0; a < 4; ++a) field.v[a] = leaf.params[a];
+						start = shape == ShapePrograms;
+						mode  = Stepping;
+						break;
+					}
+					t = fmaxf(cell.exit, t) + nudge(t);
+					++step;
+					if (over()) break;
+				}
+			}
+			if (mode == Stepping && !start) {
+				// one branch an end: a ray that skims the ground takes tens of
+				// thousands of these steps alone in its warp, each a chain
+				float p[3]     = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				bool in        = true, moved = true;
+				uint32_t turns = kMovesPerTurn;
+#pragma unroll 1
+				do {
+					const uint32_t axis = shape >> kShapeAxisShift & 3u;
+					float value         = axisValue(axis == 0 ? p[0] : axis == 1 ? p[1] : p[2], shape >> kShapeSideShift, field);
+					if (shape == ShapeSphere) value = sphereValue(p[0], p[1], p[2], field);
+					const float go = within ? fabsf(value) : value;
+					whole          = go < tolerance(p);
+					least          = value;
+					second         = within ? go : 3.0e38f; // the one program's value, its own second
+					const float on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
+					moved          = whole || on != t;
+					t              = whole ? t : on;
+					step += whole ? 0u : 1u;
+					programSteps += cost;
+					for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
+					in = inside(cell.wall, p, d);
+				} while (!whole & moved & in & (step < stepLimit) & (t <= up) & (--turns != 0u));
+				if (!whole) {
+					if (!moved) { // too small a step to move: so would be every one to the limit
+						programSteps += (stepLimit - step) * cost;
+						step = stepLimit;
+					}
+					if (!over() && !in) mode = Locating;
+				}
+			}
+		}
+		// a march step whose value is worked out: stop on the surface or go on by it
+		if (whole) {
+			const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+			const float tol  = tolerance(p);
+			const float go   = within ? second : least;
+			float on         = t;
+			uint32_t more    = 0; // program steps past the cell's own
+			++step;
+			if (!(go < tol)) {
+				on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
+			} else {
 				const GpuLeaf leaf = w.leaves[cell.leaf];
-				exitT              = cellExitBy(o, inv, cell);
-				if (leaf.occupancy == Empty || leaf.count == 0) {
-					t = fmaxf(exitT, t) + nudge(t);
-					++step;
-					if (++skipped < kCellsPerTurn) continue;
-					break; // the next turn goes on locating
+				const Field f { least, index, leaf.count, leaf.first };
+				const float3 at = make_float3(p[0], p[1], p[2]), along = make_float3(d[0], d[1], d[2]);
+				if (!within) {
+					const float big = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
+					const bool tied = second - least <= 2e-6f * (1.0f + big);
+					const uint32_t winner = tied ? winnerAt(w, at, along, f, slots) : index;
+					done(HitState { 1, t, f.first, winner, step });
+				} else {
+					// sphereFromInside: stand on the nearest surface and read the field past it
+					const float inset = 2.0f * tol, past = t + inset;
+					const InsideStop stop = insideStop(w, args.objectMaterial, args.rays[ray].within, at, make_float3(o[0] + d[0] * past, o[1] + d[1] * past, o[2] + d[2] * past),
+					                                   along, f, slots);
+					programSteps += stop.steps;
+					more = stop.steps;
+					if (stop.kind == 0) on = past;
+					else done(HitState { stop.kind, t, stop.first, stop.index, step });
 				}
-				first   = leaf.first;
-				count   = leaf.count;
-				k       = 0;
-				least   = 3.0e38f;
-				second  = 3.0e38f;
-				nearest = 3.0e38f;
-				index   = 0;
-				code       = w.march + leaf.march;
-				length     = leaf.marchCount;
-				resultSlot = leaf.marchSlot;
-				pc         = 0;
-				next       = code[0];
-				mode       = Evaluating;
-				setPoint(slots, stride, p);
-				break;
+			}
+			if (mode != Fetch) {
+				if (on == t && step < stepLimit) { // as above
+					const GpuLeaf leaf = w.leaves[cell.leaf];
+					for (uint32_t k = 0; k < leaf.count; ++k) more += w.programs[leaf.first + k].marchSteps;
+					programSteps += (stepLimit - step) * more;
+					step = stepLimit;
+				}
+				t = on;
+				if (!over()) {
+					const float q[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+					const bool in    = inside(cell.wall, q, d);
+					start            = in && shape == ShapePrograms;
+					mode             = in ? Stepping : Locating;
+				}
 			}
 		}
-
-		// a few program steps; each step's code is loaded a step ahead
-		if (mode == Evaluating) {
-			for (uint32_t u = 0; u < kStepsPerTurn; ++u) {
-				const MarchStep s = next;
-				MarchParams q {};
-				if (fusedStep(s)) q = paramsAt(code + ++pc);
-				if (pc + 1 < length) next = code[pc + 1];
-				marchStep(s, q, slots, stride);
-				if (++pc == length) break;
-			}
-			if (pc == length) {
-				const float v = slots[resultSlot * stride];
-				programSteps += length;
-				if (v < least) {
-					second = least;
-					least  = v;
-					index  = k;
-				} else if (v < second) {
-					second = v;
-				}
-				nearest = fminf(nearest, fabsf(v));
-				if (++k < count) {
-					const GpuProgram g = w.programs[first + k];
-					code       = w.march + g.march;
-					length     = g.marchCount;
-					resultSlot = g.marchSlot;
-					pc         = 0;
-					next       = code[0];
-				} else {
-					// the march step: stop on the surface or go on by the field
-					const float tol = tolerance(p);
-					++step;
-					mode = Locating;
-					if (!inside) {
-						if (least < tol) {
-							Field f;
-							f.least = least;
-							f.index = index;
-							f.count = count;
-							f.first = first;
-							const float big  = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
-							const bool tied  = second - least <= 2e-6f * (1.0f + big);
-							const uint32_t winner = tied ? winnerAt(w, o, d, t, f, slots, stride) : index;
-							done(HitState { 1, t, first, winner, step });
-						} else {
-							t = fminf(t + least, fmaxf(exitT, t) + nudge(t));
-						}
-					} else if (nearest < tol) {
-						// sphereFromInside: stand on the nearest surface and read the field past it
-						Field f;
-						f.least = least;
-						f.index = index;
-						f.count = count;
-						f.first = first;
-						const float inset   = 2.0f * tol;
-						const InsideStop at = insideStop(w, args.objectMaterial, medium, o, d, t, inset, f, cell, slots, stride, programSteps);
-						if (at.kind == 0) t += inset;
-						else done(HitState { at.kind, t, at.first, at.index, step });
-					} else {
-						t = fminf(t + nearest, fmaxf(exitT, t) + nudge(t));
-					}
-				}
-			}
+		if (start) {
+			const GpuLeaf leaf = w.leaves[cell.leaf];
+			pc    = leaf.march;
+			end   = leaf.march + leaf.marchCount;
+			order = leaf.count;
+			cost  = leaf.marchSteps;
+			memcpy(&next, leaf.params, sizeof next);
+			field.v[0] = 3.0e38f;
+			field.v[1] = 3.0e38f;
+			mode       = Evaluating;
 		}
 	}
 	if (args.counters) {

@@ -33,26 +33,37 @@ enum Op : uint8_t {
 // point and the step's immediate.  Every other reference operation is a
 // rare step (kMarchRare + opcode) over slots a, b, c.
 //
-// The runs of steps that signed distances are made of are fused further, each
-// into one step of two units (the second its parameters) that rounds at
-// every point the single steps round at, so its value is theirs to the bit:
-//  - FormAxis: a coordinate's distance to a slab, p - c, |p - c| or -(p - c),
-//    then - h, + r, - e (a term left out is an exact zero);
-//  - FormSphere: sqrt((x - cx)^2 + (y - cy)^2 + (z - cz)^2) - r;
-//  - FormNorm: the root of two or three slots' sum of squares (each squared
-//    whole or its positive part, added by itself or by a fused multiply-add),
-//    with the inside term min(m, 0) of a box and the rounding - e.
-// A rounded box of 19 steps is three axes and a norm.  On config 2 the march
-// runs 105 single steps a ray and 42 fused ones.
+// The runs of steps that signed distances are made of are fused further, into
+// steps of two or three units that round at every point the single steps
+// round at, so their values are theirs to the bit:
+//  - FormPrimitive: up to three slabs of the point, each p - c, |p - c| or
+//    -(p - c), then - h and + r; their sum of squares' root, one's positive
+//    part, or the one slab itself; a box's inside term; and - e.  A plane, a
+//    sphere, and a rounded box with the faces, edges and corners a cut leaves
+//    of it are one step each, the same operations for all of them, so a warp
+//    whose lanes are at different ones does not split;
+//  - FormNorm: such a root over slots, where other steps read the slabs too
+//    or make them;
+//  - FormRepeat: a coordinate taken into the middle cell of a repetition,
+//    x - s * floor(x / s + o).
+// 98% of the programs the march runs on config 2 and the city are primitives
+// alone, joined by the post operations.
 enum MarchPost : uint8_t { PostNone, PostSqrt, PostAbs, PostPosSq, PostMin, PostMax, PostSminK };
-enum MarchForm : uint8_t { FormFma = 0, FormAxis = 8, FormSphere = 16, FormNorm = 24 }; // op = form + post
-constexpr uint8_t kMarchPostMask = 7, kMarchFormMask = 24;
+enum MarchForm : uint8_t { FormFma = 0, FormAxis = 8, FormPrimitive = 16, FormNorm = 24, FormRepeat = 32 }; // op = form + post; FormAxis: in the lowering alone
+constexpr uint8_t kMarchPostMask = 7, kMarchFormMask = 56;
 constexpr uint8_t kMarchRare = 64;
 enum AxisSide : uint8_t { SideNone, SideAbs, SideNegative };
-// FormNorm's flags: which terms are squared by their positive part, which are
-// added by a fused multiply-add, a third term, an inside term in slot m, and
-// that the inside term is the terms' own maximum
-enum NormFlag : uint8_t { NormPositive0 = 1, NormPositive1 = 2, NormPositive2 = 4, NormFused1 = 8, NormFused2 = 16, NormThree = 32, NormInside = 64, NormInsideMax = 128 };
+// The terms of a root (FormNorm, FormPrimitive): which are in the sum, which
+// are squared by their positive part, which are added by a fused multiply-add
+enum SumFlag : uint8_t { SumHas0 = 1, SumHas1 = 2, SumHas2 = 4, SumPositive0 = 8, SumPositive1 = 16, SumPositive2 = 32, SumFused1 = 64, SumFused2 = 128 };
+// FormNorm's m where it has no inside term
+constexpr uint8_t kNoInside = 255;
+// FormPrimitive's m: the slab itself; the sum's one term's positive part; an
+// inside term, and that it spans a third term; the h and r unit follows; the
+// post operation's w is the step before's result; the result is read from its slot
+enum PrimitiveFlag : uint8_t { PrimPlain = 1, PrimSingle = 2, PrimInside = 4, PrimThird = 8, PrimSized = 16, PrimPrevious = 32, PrimStored = 64 };
+// FormPrimitive's a, b, c: bits 0-1 the axis, bits 2-3 its AxisSide
+constexpr uint8_t kTermSideShift = 2;
 enum MarchSlot : uint8_t { SlotZero, SlotOne, SlotMinusOne, SlotX, SlotY, SlotZ, SlotImm, kMarchFirstSlot };
 
 struct alignas(16) MarchStep {
@@ -60,14 +71,14 @@ struct alignas(16) MarchStep {
 	uint8_t dst; // slot of the result
 	uint8_t a, b, c;
 	uint8_t w;   // the post operation's second operand (min, max, smooth minimum)
-	uint8_t m;     // FormNorm: the inside term's slot
-	uint8_t flags; // FormAxis: AxisSide; FormNorm: NormFlag
-	float value;   // the immediate (SlotImm); a smooth minimum's radius
-	float quarter; // 0.25 / radius of a smooth minimum
+	uint8_t m;     // FormNorm: the inside term's slot; FormPrimitive: PrimitiveFlag
+	uint8_t flags; // FormNorm, FormPrimitive: SumFlag
+	float value;   // the immediate (SlotImm); a smooth minimum's radius; FormRepeat: s
+	float quarter; // 0.25 / radius of a smooth minimum; FormRepeat: o
 };
 static_assert(sizeof(MarchStep) == 16, "MarchStep is 16 bytes");
-// A fused step's second unit: FormAxis c, h, r, e; FormSphere the centre and
-// the radius; FormNorm e.
+// A fused step's second unit: FormNorm e; FormPrimitive the terms' c and e,
+// and where PrimSized a third, the terms' h and r.
 struct alignas(16) MarchParams {
 	float v[4];
 };
@@ -108,8 +119,7 @@ struct alignas(16) GpuProgram {
 	uint16_t marchCount; // units of the march form (a fused step takes two)
 	uint32_t object;     // index into the scene's object programs
 	uint32_t march;      // first MarchStep of the march form
-	uint8_t marchSlot;   // slot of the result in the march form
-	uint8_t marchSlots;
+	uint16_t marchSlots; // slots the march form uses
 	uint16_t marchSteps; // single steps the march form stands for (what the counters count)
 	uint32_t pad1[2];
 };
@@ -117,31 +127,47 @@ static_assert(sizeof(GpuProgram) == 32, "GpuProgram is 32 bytes");
 
 enum Occupancy : uint8_t { Empty = 0, Filled = 1, Surface = 2 };
 
+// A leaf.  An empty one, or one whose one program is a single axis or sphere
+// (on config 2, 54% and 34% of the march's steps; on a ray that skims the
+// ground, all of them), is marched from the record itself, in registers: an
+// empty leaf is an axis infinitely far from its slab.
+enum LeafShape : uint8_t { ShapeAxis = 0, ShapeSphere = 1, ShapePrograms = 2, ShapeEmpty = 3 }; // bits 0-1
+constexpr uint8_t kShapeMask = 3, kShapeAxisShift = 2, kShapeSideShift = 4; // an axis: bits 2-3 which, 4-5 its AxisSide
 struct alignas(16) GpuLeaf {
 	uint32_t first;     // first GpuProgram
-	uint16_t count;     // kept programs
-	uint8_t occupancy;
-	uint8_t slots;      // most slots of its programs
+	uint8_t count;      // kept programs
+	uint8_t pad0;
+	uint8_t shape;      // LeafShape
+	uint8_t pad1;
 	// the first program's march form, read with the leaf
 	uint32_t march;
 	uint16_t marchCount;
-	uint8_t marchSlot;
-	uint8_t pad;
+	uint16_t marchSteps;
+	// of an axis c, h, r, e; of a sphere its centre and radius; of programs the
+	// first one's first unit (MarchStep)
+	float params[4];
 };
-static_assert(sizeof(GpuLeaf) == 16, "GpuLeaf is 16 bytes");
+static_assert(sizeof(GpuLeaf) == 32, "GpuLeaf is 32 bytes");
 
-// The octree cut across at one level: for each cell of the uniform grid of
-// that level, the node value there (first child, or ~leaf) and its level,
-// less than the grid's where a leaf above it covers the cell.  A point is
-// located by its grid cell (an estimate from its coordinates, set right
-// against the grid's walls), one load, and the descent below it.  The walls
-// are the descent's own midpoints, 0.5 * (lo + hi) level by level in FP32,
-// so a point lands in the cell the descent from the root would give it.
-struct GridCell {
-	int32_t node;
-	uint32_t level;
-};
-constexpr uint32_t kGridLevel = 6;
+// Locating a point.  The tree's walls down to its finest level (kMostFine at
+// most) are tabled per axis: the descent's own midpoints, 0.5 * (lo + hi)
+// level by level in FP32, so a point's place among them, whose bits are the
+// descent's choices, is the place the descent from the root would give it.
+// The place is estimated by one multiply-add, a quarter of a place low, and
+// set right by the one wall above it; the build checks that the estimate is
+// never off by more (fineLevelOf) and tables fewer levels where it would be.
+// The octree cut across at kGridLevel gives what is there by one load, and
+// below it bricks of 4 x 4 x 4 give two levels by one load each (most steps of
+// a march end in an empty cell, whose size is all it needs to know: three
+// dependent loads for a cell of level 11, where child by child and its leaf's
+// record were six).  Leaves below the finest tabled level go on by midpoints.
+//
+// A grid or brick entry: a leaf (kEntryLeaf; kEntryEmpty where it is empty;
+// its level in four bits, its index in 26); else above the finest tabled level
+// a brick, and there the first child of an octree node.
+constexpr uint32_t kEntryLeaf = 1u << 31, kEntryEmpty = 1u << 30, kEntryLevelShift = 26, kEntryIndex = (1u << 26) - 1u;
+constexpr uint32_t kBrick = 64; // entries a brick, x fastest
+constexpr uint32_t kGridLevel = 7, kMostFine = 12;
 
 // Everything the trace kernel reads, as device pointers.
 struct DeviceWorld {
@@ -152,10 +178,11 @@ struct DeviceWorld {
 	const MarchStep* march;
 	const SsaOps* ssa;
 	const uint32_t* leaf_material;
-	const GridCell* grid; // (2^gridLevel)^3 cells, x fastest; null: descend from the root
-	const float* gridWalls; // per axis 2^gridLevel + 1 walls
-	uint32_t gridLevel;
-	float gridScale[3];   // 2^gridLevel / size
+	const uint32_t* grid;   // the entries of the (2^gridLevel)^3 cells, x fastest
+	const uint32_t* bricks;
+	const float* walls;   // per axis 2^fineLevel + 1 walls
+	uint32_t gridLevel, fineLevel;
+	float scale[3], bias[3]; // a point's place: p * scale + bias, rounded down
 	float lower[3];
 	float size[3];
 	uint32_t leaf_count;

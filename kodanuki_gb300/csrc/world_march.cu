@@ -30,7 +30,7 @@ extern "C" kdn_status kdn_world_march(kdn_ctx* handle, uint64_t i, const float* 
 	for (uint32_t k = 0; k < leaf.count; ++k) {
 		const kdn::GpuProgram& g = ctx->flat.programs[leaf.first + k];
 		const kdn::MarchStep* code = ctx->flat.march.data() + g.march;
-		for (uint32_t j = 0; j < n; ++j) values[size_t(k) * n + j] = kdn::evalSlots(code, g.marchCount, g.marchSlot, slots.data(), 1, points + 3 * size_t(j));
+		for (uint32_t j = 0; j < n; ++j) values[size_t(k) * n + j] = kdn::evalSlots(code, g.marchCount, slots.data(), 1, points + 3 * size_t(j));
 	}
 	return KDN_OK;
 }
@@ -47,15 +47,11 @@ extern "C" kdn_status kdn_world_locate(kdn_ctx* handle, const float* points, uin
 	kdn::DeviceWorld w {};
 	w.nodes     = ctx->flat.nodes.data();
 	w.grid      = ctx->gridCells.data();
-	w.gridWalls = ctx->walls.data();
-	w.gridLevel = kdn::kGridLevel;
-	for (int a = 0; a < 3; ++a) {
-		w.lower[a]     = ctx->lowerF[a];
-		w.size[a]      = ctx->sizeF[a];
-		w.gridScale[a] = float(double(1u << kdn::kGridLevel) / double(w.size[a]));
-	}
+	w.bricks    = ctx->bricks.data();
+	w.walls     = ctx->walls.data();
+	ctx->setLocating(w);
 	for (uint32_t j = 0; j < n; ++j) {
-		by_grid[j]    = kdn::locate(w, points + 3 * size_t(j)).leaf;
+		by_grid[j]    = kdn::locate(w, points + 3 * size_t(j));
 		by_descent[j] = kdn::descendFromRoot(w, points + 3 * size_t(j));
 	}
 	return KDN_OK;

@@ -1,8 +1,8 @@
 """The fused steps of the march form (world.h MarchForm) against a plain
-double evaluation of the programs they stand for: slabs, spheres, and rounded
-boxes, alone and joined, kept whole (no cut) and cut by the cells of a small
-octree, where a box loses axes, its corners and edges square an axis whole,
-and an inside term stays or goes.
+double evaluation of the programs they stand for: slabs, spheres, rounded
+boxes and a repetition, alone and joined, kept whole (no cut) and cut by the
+cells of a small octree, where a box loses axes, its corners and edges square
+an axis whole, and an inside term stays or goes.
 
 The tolerance is FP32's: a program of n steps over values below V rounds each
 step by at most V * 2^-24 and the root of a sum of squares loses at most the
@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from helpers import host_backend
-from test_march_form import ABS, ADD, CONSTANT, MAX, MIN, MUL, NEG, POSSQ, PX, SMIN, SQRT, SUB, evaluate
+from test_march_form import ABS, ADD, CONSTANT, DIV, FLOOR, MAX, MIN, MUL, NEG, POSSQ, PX, SMIN, SQRT, SUB, evaluate
 
 import kodanuki_gb300 as K
 from kodanuki_gb300.scene import STEP_DTYPE
@@ -53,6 +53,11 @@ class Program:
         inside = self.op(MIN, most, self.const(0.0))
         return self.op(SUB, self.op(ADD, self.op(SQRT, total), inside), self.const(round_))
 
+    def repeated(self, axis, centre, period):
+        u = self.op(SUB, self.op(PX + axis), self.const(centre))
+        k = self.op(FLOOR, self.op(ADD, self.op(DIV, u, self.const(period)), self.const(0.5)))
+        return self.op(SUB, u, self.op(MUL, self.const(period), k))
+
     def slab(self, axis, centre, half, negative=False):
         u = self.op(SUB, self.op(PX + axis), self.const(centre))
         u = self.op(NEG, u) if negative else self.op(ABS, u)
@@ -82,6 +87,11 @@ def programs():
     p = Program()
     a, b = p.box((0.0, 0.0, 0.0), (0.5, 0.4, 0.45), 0.03), p.sphere((0.4, 0.3, 0.2), 0.3)
     p.op(MAX, a, p.op(NEG, b))
+    out.append(p)
+    p = Program()  # balls in a row: a repeated coordinate beside two plain ones
+    d = [p.repeated(0, 0.05, 0.4)] + [p.op(SUB, p.op(PX + k), p.const(0.1 * k)) for k in (1, 2)]
+    total = p.op(ADD, p.op(MUL, d[2], d[2]), p.op(ADD, p.op(MUL, d[0], d[0]), p.op(MUL, d[1], d[1])))
+    p.op(SUB, p.op(SQRT, total), p.const(0.15))
     out.append(p)
     return out
 
@@ -117,6 +127,11 @@ def test_fused_steps_match_programs(build):
                 # away from a root of a sum near zero (see above)
                 roots = [evaluate(cut[:k + 1], k, pts.astype(np.float64)) for k in range(len(cut)) if cut[k]["opcode"] == SQRT]
                 clear = np.all([(r > 1e-2) | (r == 0) for r in roots], axis=0) if roots else np.ones(len(pts), bool)
+                # and from a floor's step, where FP32 and double may take either side
+                for k in range(len(cut)):
+                    if cut[k]["opcode"] == FLOOR:
+                        a = evaluate(cut[:k], int(cut[k]["a"]), pts.astype(np.float64))
+                        clear &= np.abs(a - np.round(a)) > 1e-5
                 assert np.abs(got[0] - want)[clear].max(initial=0.0) <= 3.1e-5
                 checked += int(clear.sum())
         finally:
