@@ -21,12 +21,14 @@ namespace {
 constexpr int kTraceBlock = 128;
 // A thread's register slots are a column of shared memory, one float a slot.
 constexpr uint32_t kStride = kTraceBlock;
-// cells a turn takes a ray through while they are empty, march steps inside a
-// shaped cell (world.h LeafShape) and program steps, before the warp looks again at what most of its
-// rays wait for
-constexpr uint32_t kCellsPerTurn = 3;
-constexpr uint32_t kMovesPerTurn = 8;
-constexpr uint32_t kStepsPerTurn = 4;
+// rays of a warp that may wait at their ends before the warp sees to them
+constexpr uint32_t kWaiting = 8;
+// steps a ray takes in a shaped cell (world.h LeafShape), and program steps,
+// a turn (2 to 8 and 1 to 4 measured within 3%); with kFew rays in hand, kAlone
+constexpr uint32_t kMovesPerTurn = 4, kStepsPerTurn = 2;
+constexpr uint32_t kFew = 4, kAlone = 64;
+// steps worked out at once where a ray is seen to stay in its cell
+constexpr uint32_t kRun = 8;
 
 __device__ __forceinline__ float slopeOf(float part) {
 	const float tiny = 1e-12f;
@@ -155,11 +157,16 @@ __device__ __noinline__ InsideStop insideStop(const DeviceWorld& w, const uint32
 // The march as a step machine.  Each thread holds one ray at a time.  A ray
 // waits to be located, or to step in a cell whose field its leaf record holds
 // (empty, or a single slab or sphere: a few operations in registers), or for
-// the programs of its cell, a few of their steps at a time; every turn the
-// warp does what most of its rays wait for.  A ray that ends takes the next
-// ray of the launch (one atomic a warp).
-enum LaneMode : uint32_t { Fetch = 0, Locating = 1, Stepping = 2, Evaluating = 3, Finished = 4 };
+// the programs of its cell, a step of theirs at a time; every turn the warp
+// does the one thing most of its rays wait for.  Rays that have landed or
+// ended wait until there are several, and the ended take the next rays of the
+// launch (one atomic a warp).
+// A mode's number is its count's place in the warp's sum of them.
+enum LaneMode : uint32_t { Locating = 1, Stepping = 1 << 8, Evaluating = 1 << 16, Fetch = 1 << 24, Landed = 3 << 24, Finished = 5 << 24 };
 
+// Five blocks an SM (96 registers) hold the machine's state in registers: six
+// spill it (config 2's frame 550 against 489 ms), four hide less of the
+// loads' latency (492 against 475 ms).
 __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_constant__ TraceArgs args) {
 	extern __shared__ float slotMemory[];
 	const DeviceWorld& w = args.world;
@@ -180,7 +187,7 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 	}
 	uint32_t mode = Fetch;
 	uint32_t ray  = 0;
-	float o[3], d[3], inv[3];
+	float o[3] = { 0.0f, 0.0f, 0.0f }, d[3] = { 0.0f, 0.0f, 0.0f }, inv[3] = { 0.0f, 0.0f, 0.0f };
 	float t = 0.0f, up = 0.0f;
 	bool within   = false; // the ray started inside a solid
 	uint32_t step = 0;
@@ -216,72 +223,171 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 		return true;
 	};
 
+	// a ray goes on from t to on, its march step taken: to the end of its march,
+	// on in its cell, or out of it.  A step too small to move it would be taken
+	// again to the limit: cost, what one adds to the program step count.
+	auto goOn = [&](float on, uint32_t stepCost) {
+		if (on == t) {
+			programSteps += (stepLimit - step) * stepCost;
+			step = stepLimit;
+		}
+		t = on;
+		if (over()) return;
+		const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+		mode             = inside(cell.wall, p, d) ? Stepping : Locating;
+	};
+	// a ray starts on the programs of its cell
+	auto start = [&](const GpuLeaf& leaf) {
+		pc    = leaf.march;
+		end   = leaf.march + leaf.marchCount;
+		order = leaf.count;
+		cost  = leaf.marchSteps;
+		memcpy(&next, leaf.params, sizeof next);
+		field.v[0] = 3.0e38f;
+		field.v[1] = 3.0e38f;
+		mode       = Evaluating;
+	};
+	uint32_t finished = 0; // lanes without a ray, the launch's all taken
+
 	for (;;) {
-		// take new rays, one atomic a warp
-		const bool want     = mode == Fetch;
-		const unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
-		if (mask) {
-			uint32_t base = 0;
-			const int leader = __ffs(mask) - 1;
-			if (int(lane) == leader) base = atomicAdd(args.fetch, uint32_t(__popc(mask)));
-			base = __shfl_sync(0xFFFFFFFFu, base, leader);
-			if (want) {
-				ray = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
-				if (ray >= n) {
-					mode = Finished;
+		const uint32_t modes      = __reduce_add_sync(0xFFFFFFFFu, mode);
+		const uint32_t locating   = modes & 0xFFu, stepping = modes >> 8 & 0xFFu, evaluating = modes >> 16 & 0xFFu;
+		const uint32_t busy       = locating + stepping + evaluating;
+		const uint32_t waiting    = 32u - busy - finished;
+		if (waiting >= kWaiting || waiting > busy) {
+			if (mode == Landed) {
+				// field and order hold what the march step came to: the least of the
+				// cell's programs, the second least (from inside, the least magnitude)
+				// and the least's index
+				const GpuLeaf leaf = w.leaves[cell.leaf];
+				const float p[3]   = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				const Field f { field.v[0], order >> 16, leaf.count, leaf.first };
+				const float3 at = make_float3(p[0], p[1], p[2]), along = make_float3(d[0], d[1], d[2]);
+				if (!within) {
+					const float big = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
+					const bool tied = field.v[1] - field.v[0] <= 2e-6f * (1.0f + big);
+					const uint32_t winner = tied ? winnerAt(w, at, along, f, slots) : f.index;
+					done(HitState { 1, t, f.first, winner, step });
 				} else {
-					if (ray >= n1) ray = args.second + (ray - n1);
-					const kdn_ray r = args.rays[ray];
-					within          = r.inside != 0;
-					for (int a = 0; a < 3; ++a) {
-						o[a]   = r.origin[a];
-						d[a]   = r.direction[a];
-						inv[a] = slopeOf(d[a]);
-					}
-					float lo = 0.0f;
-					up       = r.far;
-					for (int a = 0; a < 3; ++a) {
-						const float x = (w.lower[a] - o[a]) * inv[a];
-						const float y = (w.lower[a] + w.size[a] - o[a]) * inv[a];
-						lo            = fmaxf(lo, fminf(x, y));
-						up            = fminf(up, fmaxf(x, y));
-					}
-					t    = lo;
-					step = 0;
-					// a carried ray goes on where its march stood
-					if (args.carry != nullptr && (r.pad_[0] & kRayResumes)) {
-						const uint2 c = args.carry[ray];
-						t             = __uint_as_float(c.x);
-						step          = c.y;
+					// sphereFromInside: stand on the nearest surface and read the field past it
+					const float inset = 2.0f * tolerance(p), past = t + inset;
+					const InsideStop stop = insideStop(w, args.objectMaterial, args.rays[ray].within, at, make_float3(o[0] + d[0] * past, o[1] + d[1] * past, o[2] + d[2] * past),
+					                                   along, f, slots);
+					programSteps += stop.steps;
+					if (stop.kind == 0) {
+						uint32_t each = stop.steps;
+						if (past == t) {
+							for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
+						}
+						goOn(past, each);
+						if (mode == Stepping) mode = Locating; // the cell's field is to be read again
 					} else {
-						++traced; // a segment is counted once, in the launch that starts it
+						done(HitState { stop.kind, t, stop.first, stop.index, step });
 					}
-					stepLimit = min(args.maxSteps, step + allowance);
-					marchSteps -= step;
-					if (up < lo) done(HitState { 0, t, kNoLeaf, 0, step });
-					else if (!over()) mode = Locating;
 				}
 			}
-		}
-		const int locating   = __popc(__ballot_sync(0xFFFFFFFFu, mode == Locating));
-		const int stepping   = __popc(__ballot_sync(0xFFFFFFFFu, mode == Stepping));
-		const int evaluating = __popc(__ballot_sync(0xFFFFFFFFu, mode == Evaluating));
-		if (locating + stepping + evaluating == 0) {
-			if (__all_sync(0xFFFFFFFFu, mode == Finished)) break;
+			// take new rays, one atomic a warp
+			const unsigned mask = __ballot_sync(0xFFFFFFFFu, mode == Fetch);
+			if (mask) {
+				uint32_t base = 0;
+				const int leader = __ffs(mask) - 1;
+				if (int(lane) == leader) base = atomicAdd(args.fetch, uint32_t(__popc(mask)));
+				base = __shfl_sync(0xFFFFFFFFu, base, leader);
+				if (mode == Fetch) {
+					ray = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
+					if (ray >= n) {
+						mode = Finished;
+					} else {
+						if (ray >= n1) ray = args.second + (ray - n1);
+						const kdn_ray r = args.rays[ray];
+						within          = r.inside != 0;
+						for (int a = 0; a < 3; ++a) {
+							o[a]   = r.origin[a];
+							d[a]   = r.direction[a];
+							inv[a] = slopeOf(d[a]);
+						}
+						float lo = 0.0f;
+						up       = r.far;
+						for (int a = 0; a < 3; ++a) {
+							const float x = (w.lower[a] - o[a]) * inv[a];
+							const float y = (w.lower[a] + w.size[a] - o[a]) * inv[a];
+							lo            = fmaxf(lo, fminf(x, y));
+							up            = fminf(up, fmaxf(x, y));
+						}
+						t    = lo;
+						step = 0;
+						// a carried ray goes on where its march stood
+						if (args.carry != nullptr && (r.pad_[0] & kRayResumes)) {
+							const uint2 c = args.carry[ray];
+							t             = __uint_as_float(c.x);
+							step          = c.y;
+						} else {
+							++traced; // a segment is counted once, in the launch that starts it
+						}
+						stepLimit = min(args.maxSteps, step + allowance);
+						marchSteps -= step;
+						if (up < lo) done(HitState { 0, t, kNoLeaf, 0, step });
+						else if (!over()) mode = Locating;
+					}
+				}
+			}
+			finished = __popc(__ballot_sync(0xFFFFFFFFu, mode == Finished));
+			if (finished == 32) break;
 			continue;
 		}
-		// a march step whose value is worked out: the least of the cell's
-		// programs, the second least (from inside, the least magnitude), the least's index
-		bool whole     = false;
-		float least    = 0.0f, second = 0.0f;
-		uint32_t index = 0;
-		bool start     = false; // a ray starts on its cell's programs
-		if (evaluating > locating && evaluating > stepping) {
-			if (mode == Evaluating) {
-				// a few program steps; each step's code is loaded a step ahead
-				const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+		if (evaluating >= locating && evaluating >= stepping) {
+			if (mode == Evaluating && busy <= kFew) {
+				// few rays in hand: whole march steps at a time, each as soon as the
+				// one before is done (a ray that skims a box takes thousands; the
+				// turns above cost one 480 ns a step, these 200)
+				const GpuLeaf leaf = w.leaves[cell.leaf];
+				MarchStep s;
+				memcpy(&s, leaf.params, sizeof s);
+				const bool one = leaf.count == 1 && s.op == FormPrimitive && leaf.marchCount == unitsOf(s);
+				const MarchParams c = paramsAt(w.march + leaf.march + 1);
+				MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
+				if (one && s.m & PrimSized) h = paramsAt(w.march + leaf.march + 2);
+				uint32_t turns = kAlone;
 #pragma unroll 1
-				for (uint32_t u = 0; u < kStepsPerTurn; ++u) {
+				do {
+					const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+					float least = 3.0e38f, second = 3.0e38f;
+					uint32_t index = 0, each = 0;
+					if (one) {
+						least = primitiveValue(s, c, h, p[0], p[1], p[2]);
+						each  = leaf.marchSteps;
+						if (within) second = fabsf(least);
+					} else {
+#pragma unroll 1
+						for (uint32_t k = 0; k < leaf.count; ++k) {
+							const GpuProgram g = w.programs[leaf.first + k];
+							const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
+							const bool lesser  = v < least;
+							each += g.marchSteps;
+							second = within ? fminf(second, fabsf(v)) : lesser ? least : fminf(second, v);
+							least  = lesser ? v : least;
+							index  = lesser ? k : index;
+						}
+					}
+					programSteps += each;
+					++step;
+					const float go = within ? second : least;
+					if (go < tolerance(p)) {
+						field.v[0] = least;
+						field.v[1] = second;
+						order      = index << 16;
+						mode       = Landed;
+						break;
+					}
+					goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), each);
+				} while (mode == Stepping && --turns != 0u);
+				if (mode == Stepping) start(leaf);
+			} else if (mode == Evaluating) {
+				// the next step's code is loaded a step ahead
+				float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				uint32_t turns = kStepsPerTurn;
+#pragma unroll 1
+				do {
 					const MarchStep s     = next;
 					const MarchStep* unit = w.march + pc + 1;
 					pc += unitsOf(s);
@@ -292,15 +398,12 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 						setPoint(slots, kStride, p);
 						last = marchStep(s, unit, slots, kStride);
 					}
-					if (pc == end) break;
-				}
-				if (pc == end) {
-					const float v = last;
+					if (pc != end) continue;
 					programSteps += cost;
 					uint32_t k        = order >> 8 & 0xFFu;
-					const bool lesser = v < field.v[0];
-					field.v[1]        = within ? fminf(field.v[1], fabsf(v)) : lesser ? field.v[0] : fminf(field.v[1], v);
-					field.v[0]        = lesser ? v : field.v[0];
+					const bool lesser = last < field.v[0];
+					field.v[1]        = within ? fminf(field.v[1], fabsf(last)) : lesser ? field.v[0] : fminf(field.v[1], last);
+					field.v[0]        = lesser ? last : field.v[0];
 					if (lesser) order = (order & 0x0000FFFFu) | k << 16;
 					if (++k < (order & 0xFFu)) {
 						const GpuProgram g = w.programs[w.leaves[cell.leaf].first + k];
@@ -309,136 +412,102 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 						order = (order & 0x00FF00FFu) | k << 8;
 						cost  = g.marchSteps;
 						next  = w.march[pc];
-					} else {
-						least  = field.v[0];
-						second = field.v[1];
-						index  = order >> 16;
-						whole  = true;
+						continue;
 					}
-				}
-			}
-		} else {
-			if (mode == Locating && locating >= stepping) {
-				// the cell of the point; an empty one is left at once, for the next
-#pragma unroll 1
-				for (uint32_t u = 0; u < kCellsPerTurn; ++u) {
-					const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-					int place[3];
-					placeOf(w, p, place);
-					const uint32_t entry = entryAt(w, place);
-					bool empty           = entry & kEntryEmpty;
-					if (entry & kEntryLeaf) {
-						const uint32_t wide = w.fineLevel - (entry >> kEntryLevelShift & 15u), row = (1u << w.fineLevel) + 1u;
-						float at[3];
-						for (int a = 0; a < 3; ++a) at[a] = __ldg(w.walls + a * row + ((uint32_t(place[a]) >> wide) + (__float_as_int(d[a]) < 0 ? 0u : 1u) << wide));
-						walledBy(cell, at, o, d, inv);
-						cell.leaf = entry & kEntryIndex;
-					} else {
-						cell  = deepCell(w, make_float3(p[0], p[1], p[2]), int32_t(entry), make_int3(place[0], place[1], place[2]), make_float3(o[0], o[1], o[2]), make_float3(d[0], d[1], d[2]), make_float3(inv[0], inv[1], inv[2]));
-						empty = w.leaves[cell.leaf].shape == ShapeEmpty;
-					}
-					if (!empty) {
-						const GpuLeaf leaf = w.leaves[cell.leaf];
-						shape              = leaf.shape;
-						cost               = leaf.marchSteps;
-						for (int a = 0; a < 4; ++a) field.v[a] = leaf.params[a];
-						start = shape == ShapePrograms;
-						mode  = Stepping;
+					// stop on the surface or go on by the value
+					const float go = within ? field.v[1] : field.v[0];
+					++step;
+					if (go < tolerance(p)) {
+						mode = Landed;
 						break;
 					}
+					const GpuLeaf leaf = w.leaves[cell.leaf];
+					const float on     = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
+					uint32_t each      = 0;
+					if (on == t) {
+						for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
+					}
+					goOn(on, each);
+					if (mode != Stepping) break;
+					start(leaf);
+					for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
+				} while (--turns != 0u);
+			}
+		} else if (locating >= stepping) {
+			if (mode == Locating) {
+				// the cell of the point; an empty one is left at once
+				const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				int place[3];
+				placeOf(w, p, place);
+				const uint32_t entry = entryAt(w, place);
+				bool empty           = entry & kEntryEmpty;
+				if (entry & kEntryLeaf) {
+					const uint32_t wide = w.fineLevel - (entry >> kEntryLevelShift & 15u), row = (1u << w.fineLevel) + 1u;
+					float at[3];
+					for (int a = 0; a < 3; ++a) at[a] = __ldg(w.walls + a * row + ((uint32_t(place[a]) >> wide) + (__float_as_int(d[a]) < 0 ? 0u : 1u) << wide));
+					walledBy(cell, at, o, d, inv);
+					cell.leaf = entry & kEntryIndex;
+				} else {
+					cell  = deepCell(w, make_float3(p[0], p[1], p[2]), int32_t(entry), make_int3(place[0], place[1], place[2]), make_float3(o[0], o[1], o[2]), make_float3(d[0], d[1], d[2]), make_float3(inv[0], inv[1], inv[2]));
+					empty = w.leaves[cell.leaf].shape == ShapeEmpty;
+				}
+				if (empty) {
 					t = fmaxf(cell.exit, t) + nudge(t);
 					++step;
-					if (over()) break;
-				}
-			}
-			if (mode == Stepping && !start) {
-				// one branch an end: a ray that skims the ground takes tens of
-				// thousands of these steps alone in its warp, each a chain
-				float p[3]     = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-				bool in        = true, moved = true;
-				uint32_t turns = kMovesPerTurn;
-#pragma unroll 1
-				do {
-					const uint32_t axis = shape >> kShapeAxisShift & 3u;
-					float value         = axisValue(axis == 0 ? p[0] : axis == 1 ? p[1] : p[2], shape >> kShapeSideShift, field);
-					if (shape == ShapeSphere) value = sphereValue(p[0], p[1], p[2], field);
-					const float go = within ? fabsf(value) : value;
-					whole          = go < tolerance(p);
-					least          = value;
-					second         = within ? go : 3.0e38f; // the one program's value, its own second
-					const float on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
-					moved          = whole || on != t;
-					t              = whole ? t : on;
-					step += whole ? 0u : 1u;
-					programSteps += cost;
-					for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
-					in = inside(cell.wall, p, d);
-				} while (!whole & moved & in & (step < stepLimit) & (t <= up) & (--turns != 0u));
-				if (!whole) {
-					if (!moved) { // too small a step to move: so would be every one to the limit
-						programSteps += (stepLimit - step) * cost;
-						step = stepLimit;
-					}
-					if (!over() && !in) mode = Locating;
-				}
-			}
-		}
-		// a march step whose value is worked out: stop on the surface or go on by it
-		if (whole) {
-			const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-			const float tol  = tolerance(p);
-			const float go   = within ? second : least;
-			float on         = t;
-			uint32_t more    = 0; // program steps past the cell's own
-			++step;
-			if (!(go < tol)) {
-				on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
-			} else {
-				const GpuLeaf leaf = w.leaves[cell.leaf];
-				const Field f { least, index, leaf.count, leaf.first };
-				const float3 at = make_float3(p[0], p[1], p[2]), along = make_float3(d[0], d[1], d[2]);
-				if (!within) {
-					const float big = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
-					const bool tied = second - least <= 2e-6f * (1.0f + big);
-					const uint32_t winner = tied ? winnerAt(w, at, along, f, slots) : index;
-					done(HitState { 1, t, f.first, winner, step });
+					over();
 				} else {
-					// sphereFromInside: stand on the nearest surface and read the field past it
-					const float inset = 2.0f * tol, past = t + inset;
-					const InsideStop stop = insideStop(w, args.objectMaterial, args.rays[ray].within, at, make_float3(o[0] + d[0] * past, o[1] + d[1] * past, o[2] + d[2] * past),
-					                                   along, f, slots);
-					programSteps += stop.steps;
-					more = stop.steps;
-					if (stop.kind == 0) on = past;
-					else done(HitState { stop.kind, t, stop.first, stop.index, step });
-				}
-			}
-			if (mode != Fetch) {
-				if (on == t && step < stepLimit) { // as above
 					const GpuLeaf leaf = w.leaves[cell.leaf];
-					for (uint32_t k = 0; k < leaf.count; ++k) more += w.programs[leaf.first + k].marchSteps;
-					programSteps += (stepLimit - step) * more;
-					step = stepLimit;
-				}
-				t = on;
-				if (!over()) {
-					const float q[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-					const bool in    = inside(cell.wall, q, d);
-					start            = in && shape == ShapePrograms;
-					mode             = in ? Stepping : Locating;
+					shape              = leaf.shape;
+					cost               = leaf.marchSteps;
+					for (int a = 0; a < 4; ++a) field.v[a] = leaf.params[a];
+					mode = Stepping;
+					if (shape == ShapePrograms) start(leaf);
 				}
 			}
-		}
-		if (start) {
-			const GpuLeaf leaf = w.leaves[cell.leaf];
-			pc    = leaf.march;
-			end   = leaf.march + leaf.marchCount;
-			order = leaf.count;
-			cost  = leaf.marchSteps;
-			memcpy(&next, leaf.params, sizeof next);
-			field.v[0] = 3.0e38f;
-			field.v[1] = 3.0e38f;
-			mode       = Evaluating;
+		} else if (mode == Stepping) {
+			// a ray that skims the ground takes tens of thousands of these steps,
+			// alone in its warp, each waiting on the one before
+			uint32_t turns      = busy <= kFew ? kAlone : kMovesPerTurn;
+			const uint32_t axis = shape >> kShapeAxisShift & 3u, side = shape >> kShapeSideShift;
+			const float oa = axis == 0 ? o[0] : axis == 1 ? o[1] : o[2], da = axis == 0 ? d[0] : axis == 1 ? d[1] : d[2];
+#pragma unroll 1
+			do {
+				const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				const bool ball  = shape == ShapeSphere;
+				const float value = ball ? sphereValue(p[0], p[1], p[2], field) : axisValue(oa + da * t, side, field);
+				const float go = within ? fabsf(value) : value, tol = tolerance(p);
+				if (!ball && t + 24.0f * go < cell.exit && (da > -0.05f || go > 64.0f * tol)) {
+					// the steps of a ray that stays in its cell: t + go each, as long as
+					// none lands (their least above the tolerance, which is greatest at an
+					// end) and the last is short of the cell's walls, the march's end and
+					// its limit, and moves; all of it as step by step, or not at all
+					float at = t, before = t, least = 3.0e38f;
+#pragma unroll
+					for (uint32_t k = 0; k < kRun; ++k) {
+						const float v = axisValue(oa + da * at, side, field);
+						least         = fminf(least, within ? fabsf(v) : v);
+						before        = at;
+						at            = at + fabsf(v);
+					}
+					const float q[3] = { o[0] + d[0] * at, o[1] + d[1] * at, o[2] + d[2] * at };
+					if (least >= fmaxf(tol, tolerance(q)) && at <= cell.exit && at <= up && at != before && step + kRun < stepLimit && inside(cell.wall, q, d)) {
+						t = at;
+						step += kRun;
+						programSteps += kRun * cost;
+						continue;
+					}
+				}
+				programSteps += cost;
+				++step;
+				if (go < tol) { // it lands: the one program's value, its own second
+					field.v[0] = value;
+					field.v[1] = within ? go : 3.0e38f;
+					order      = 0;
+					mode       = Landed;
+					break;
+				}
+				goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), cost);
+			} while (mode == Stepping && --turns != 0u);
 		}
 	}
 	if (args.counters) {
