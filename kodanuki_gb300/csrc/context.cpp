@@ -221,6 +221,7 @@ kdn_status Context::extend(const kdn_ray* rays, uint32_t n, kdn_hit* hits, cudaS
 	t.counters       = nullptr;
 	t.count          = nullptr;
 	t.fetch          = static_cast<uint32_t*>(fetch.ptr);
+	if (!check(cudaMemsetAsync(t.fetch, 0, sizeof(uint32_t), on), "clear fetch")) return KDN_CUDA_ERROR;
 	if (!check(launchTrace(t, on, smCount), "trace kernel")) return KDN_CUDA_ERROR;
 	HitArgs h;
 	h.world  = world;

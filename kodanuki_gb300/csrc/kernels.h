@@ -34,7 +34,7 @@ struct TraceArgs {
 	uint32_t maxSteps;
 	unsigned long long* counters;   // [0] march steps, [1] program steps, [2] longest march, [3] capped rays, [4] rays
 	const uint32_t* count;          // if set, the number of rays is read here on the device
-	uint32_t* fetch;                // the next ray to take; launchTrace zeroes it
+	uint32_t* fetch;                // the next ray to take: zero before the launch
 	// a second run of rays in the same arrays, from index `second` on, its
 	// count read on the device (null: none); traced in the same launch
 	const uint32_t* secondCount = nullptr;
@@ -49,6 +49,12 @@ struct TraceArgs {
 	// where set, a count that must be zero (path rays left after a frame's
 	// last round): added to counters[6], which the host checks
 	const uint32_t* left = nullptr;
+	// counts the launches after this one start from zero (null: none)
+	uint32_t* clear[2] = { nullptr, nullptr };
+	// memory the host reads meanwhile (null: none): [0] takes `turn` once the
+	// launch has begun, [1] `chunk` where it has no rays
+	volatile uint32_t* reached = nullptr;
+	uint32_t turn = 0, chunk = 0;
 };
 
 // kdn_hit.kind of a carried ray: distance is where its march stands, cell
@@ -64,6 +70,7 @@ struct HitArgs {
 	uint32_t n;
 	kdn_hit* hits;
 	const uint32_t* count;          // if set, the number of rays is read here on the device
+	uint32_t* fetch = nullptr;      // if set, the trace launch's before, left zero for the next
 };
 
 cudaError_t setTraceAttributes();

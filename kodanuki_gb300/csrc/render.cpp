@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <thread>
 
 namespace kdn {
 
@@ -80,6 +81,12 @@ struct FrameState {
 	cudaEvent_t ended[kLanes - 1] = {};   // each other lane's end of the chunks
 	cudaStream_t surfaceStream    = nullptr; // the surfaces pass
 	cudaEvent_t surfacesDone      = nullptr; // its end
+	// what each lane's trace launches tell the host meanwhile (TraceArgs::reached)
+	volatile uint32_t* reached  = nullptr;
+	uint32_t* reachedOnDevice   = nullptr;
+	// numbers of turns and chunks, going on from frame to frame so that a
+	// launch of an earlier chunk never speaks for a later one
+	uint32_t turnSerial = 0, chunkSerial = 0;
 	kdn_frame_stats stats {};
 };
 
@@ -106,6 +113,7 @@ void Context::releaseFrame() {
 		cudaStreamDestroy(f.surfaceStream);
 	}
 	if (f.surfacesDone) cudaEventDestroy(f.surfacesDone);
+	if (f.reached) cudaFreeHost(const_cast<uint32_t*>(f.reached));
 	delete frame;
 	frame = nullptr;
 }
@@ -371,6 +379,22 @@ kdn_status ensureFrame(Context* ctx, uint32_t capacity, uint32_t lineRoom) {
 	return KDN_OK;
 }
 
+// The rounds the host may be ahead of a lane's trace launches.
+constexpr int kAhead = 12;
+
+// Waits until a lane's trace launch of `turn` has begun (or the lane's stream
+// has nothing left to run, after an error).
+kdn_status reachedTurn(Context* ctx, volatile const uint32_t* reached, uint32_t turn, cudaStream_t stream) {
+	for (uint32_t spin = 1; int32_t(reached[0] - turn) < 0; ++spin) {
+		std::this_thread::yield();
+		if (spin % 256 != 0) continue;
+		const cudaError_t e = cudaStreamQuery(stream);
+		if (e == cudaSuccess) return KDN_OK;
+		if (e != cudaErrorNotReady) return ctx->check(e, "kdn_render"), KDN_CUDA_ERROR;
+	}
+	return KDN_OK;
+}
+
 kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream_t stream, bool hostOut) {
 	using namespace kdn;
 	if (!ctx->built) return ctx->fail(KDN_NOT_READY, "kdn_render: no world built (kdn_build)");
@@ -418,6 +442,7 @@ kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream
 	const uint32_t lineRoom    = ownLines ? 1u + kOwnLines : 1u;
 	const uint64_t want        = chunkPaths(ctx, uint64_t(pixels) * spp, ownLines) / kLanes;
 	const uint32_t chunkPixels = uint32_t(std::max<uint64_t>(1, (want + spp - 1) / spp));
+	const uint32_t chunks      = (pixels + chunkPixels - 1) / chunkPixels;
 	const uint32_t capacity    = chunkPixels * spp;
 	const uint32_t lineCapacity = capacity * lineRoom;
 	kdn_status s = ensureFrame(ctx, capacity, lineRoom);
@@ -761,7 +786,15 @@ kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream
 	const int rounds        = budgeted ? 2 * mainRounds : mainRounds;
 
 	// timing: one event pair around the frame, one around each trace launch
-	const uint32_t chunks = (pixels + chunkPixels - 1) / chunkPixels;
+	if (f.reached == nullptr) {
+		void* host = nullptr;
+		void* dev  = nullptr;
+		if (!ctx->check(cudaHostAlloc(&host, 2 * kLanes * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc")) return KDN_CUDA_ERROR;
+		std::memset(host, 0, 2 * kLanes * sizeof(uint32_t));
+		f.reached = static_cast<volatile uint32_t*>(host);
+		if (!ctx->check(cudaHostGetDevicePointer(&dev, host, 0), "cudaHostGetDevicePointer")) return KDN_CUDA_ERROR;
+		f.reachedOnDevice = static_cast<uint32_t*>(dev);
+	}
 	const size_t traceEvents = size_t(chunks) * size_t(rounds) * 2;
 	const size_t needEvents  = 2 + traceEvents;
 	while (f.events.size() < needEvents) {
@@ -811,6 +844,7 @@ kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream
 			t.counters       = nullptr;
 			t.count          = sq.count;
 			t.fetch          = static_cast<uint32_t*>(ctx->fetch.ptr) + kLanes;
+			if (!ctx->check(cudaMemsetAsync(t.fetch, 0, sizeof(uint32_t), on), "clear fetch")) return KDN_CUDA_ERROR;
 			if (!ctx->check(launchTrace(t, on, ctx->smCount), "surface trace kernel")) return KDN_CUDA_ERROR;
 			HitArgs h;
 			h.world  = ctx->world;
@@ -833,101 +867,134 @@ kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream
 		}
 		if (!ctx->check(cudaEventRecord(f.surfacesDone, on), "event")) return KDN_CUDA_ERROR;
 	}
-	uint32_t chunkIndex = 0;
-	for (uint32_t first = 0; first < pixels; first += chunkPixels, ++chunkIndex) {
-		const int l              = int(chunkIndex % kLanes);
-		const Lane& L            = lane[l];
-		const cudaStream_t on    = lanes[l];
-		const uint32_t chunk     = std::min(chunkPixels, pixels - first);
-		const uint32_t n         = chunk * spp;
-		const PathBuffers& LP    = L.P;
-		if (training && !ctx->check(cudaMemsetAsync(L.records, 0xFF, size_t(n) * kGuideDepth * sizeof(GuideRecord), on), "clear guide records")) return KDN_CUDA_ERROR;
-		if (!ctx->check(launchCamera(c, LP, L.Q[0], first, n, on, ctx->smCount), "camera kernel")) return KDN_CUDA_ERROR;
-		++launches;
-		if (!ctx->check(cudaMemsetAsync(L.S[0].count, 0, 4, on), "clear lines")) return KDN_CUDA_ERROR;
-		int q = 0;
+	// The chunks go round the lanes kLanes at a time, a round of each lane's
+	// after the other's, so all lanes start at once.  Most rounds past the
+	// first few have no rays left (a scattering body's path may take the
+	// collision cap's rounds, and hardly any does): each trace launch tells the
+	// host that it has begun and whether it has rays, and the host stays
+	// kAhead rounds ahead and ends a chunk whose rays have run out (a frame of
+	// 265 rounds 67 -> 25 ms).
+	for (uint32_t group = 0; group < chunks; group += kLanes) {
+		const int members = int(std::min<uint32_t>(kLanes, chunks - group));
+		int turn[kLanes]  = {};     // which of the queue pairs each lane is at
+		bool over[kLanes] = {};
+		for (int l = 0; l < members; ++l) {
+			const Lane& L         = lane[l];
+			const uint32_t first  = (group + uint32_t(l)) * chunkPixels;
+			const uint32_t n      = std::min(chunkPixels, pixels - first) * spp;
+			if (training && !ctx->check(cudaMemsetAsync(L.records, 0xFF, size_t(n) * kGuideDepth * sizeof(GuideRecord), lanes[l]), "clear guide records")) return KDN_CUDA_ERROR;
+			if (!ctx->check(launchCamera(c, L.P, L.Q[0], first, n, lanes[l], ctx->smCount), "camera kernel")) return KDN_CUDA_ERROR;
+			++launches;
+			if (!ctx->check(cudaMemsetAsync(L.S[0].count, 0, 4, lanes[l]), "clear lines") || !ctx->check(cudaMemsetAsync(L.fetch, 0, 4, lanes[l]), "clear fetch")) return KDN_CUDA_ERROR;
+		}
+		const uint32_t turns = f.turnSerial; // this group's are turns + 1 on
+		f.turnSerial += uint32_t(rounds);
+		++f.chunkSerial;
 		// each round traces the bounce's path rays and the bounce before's
 		// shadow lines in one launch; a last round traces the last lines alone
 		for (int round = 0; round < rounds; ++round) {
 			const bool last = round == rounds - 1;
-			const int nxt   = 1 - q;
-			TraceArgs t;
-			t.world          = ctx->world;
-			t.rays           = L.Q[q].rays;
-			t.n              = n;
-			t.states         = L.states;
-			t.objectMaterial = static_cast<const uint32_t*>(ctx->objectMaterial.ptr);
-			t.maxSteps       = kMarchSteps;
-			t.counters       = static_cast<unsigned long long*>(ctx->counters.ptr);
-			t.count          = last ? L.none : L.Q[q].count;
-			t.fetch          = L.fetch;
-			t.secondCount    = L.S[q].count;
-			t.second         = capacity;
-			t.carry          = L.Q[q].carry;
-			t.budget         = budgeted && round < mainRounds ? ctx->marchBudget : 0u;
-			t.left           = last ? L.Q[q].count : nullptr;
-			cudaEventRecord(f.events[ev++], on);
-			if (!ctx->check(launchTrace(t, on, ctx->smCount), "trace kernel")) return KDN_CUDA_ERROR;
-			cudaEventRecord(f.events[ev++], on);
-			++launches;
-			if (!last) {
-				HitArgs h;
-				h.world  = ctx->world;
-				h.rays   = L.Q[q].rays;
-				h.states = L.states;
-				h.n      = n;
-				h.hits   = L.hits;
-				h.count  = L.Q[q].count;
-				if (!ctx->check(launchHits(h, on, ctx->smCount), "hit kernel")) return KDN_CUDA_ERROR;
+			for (int l = 0; l < members; ++l) {
+				if (over[l]) continue;
+				const Lane& L            = lane[l];
+				const cudaStream_t on    = lanes[l];
+				const uint32_t n         = std::min(chunkPixels, pixels - (group + uint32_t(l)) * chunkPixels) * spp;
+				const PathBuffers& LP    = L.P;
+				const int q = turn[l], nxt = 1 - q;
+				if (round > kAhead) {
+					if ((s = reachedTurn(ctx, f.reached + 2 * l, turns + uint32_t(round - kAhead), on)) != KDN_OK) return s;
+				}
+				if (round > 0 && f.reached[2 * l + 1] == f.chunkSerial) {
+					over[l] = true;
+					continue;
+				}
+				TraceArgs t;
+				t.world          = ctx->world;
+				t.rays           = L.Q[q].rays;
+				t.n              = n;
+				t.states         = L.states;
+				t.objectMaterial = static_cast<const uint32_t*>(ctx->objectMaterial.ptr);
+				t.maxSteps       = kMarchSteps;
+				t.counters       = static_cast<unsigned long long*>(ctx->counters.ptr);
+				t.count          = last ? L.none : L.Q[q].count;
+				t.fetch          = L.fetch;
+				t.secondCount    = L.S[q].count;
+				t.second         = capacity;
+				t.carry          = L.Q[q].carry;
+				t.budget         = budgeted && round < mainRounds ? ctx->marchBudget : 0u;
+				t.left           = last ? L.Q[q].count : nullptr;
+				t.clear[0]       = L.S[nxt].count;
+				t.clear[1]       = last ? nullptr : L.Q[nxt].count;
+				t.reached        = f.reachedOnDevice + 2 * l;
+				t.turn           = turns + uint32_t(round) + 1u;
+				t.chunk          = f.chunkSerial;
+				cudaEventRecord(f.events[ev++], on);
+				if (!ctx->check(launchTrace(t, on, ctx->smCount), "trace kernel")) return KDN_CUDA_ERROR;
+				cudaEventRecord(f.events[ev++], on);
 				++launches;
-				if (guiding && round < kGuideDepth) {
-					GuideQueue gq;
-					gq.hits          = L.hits;
-					gq.rays          = L.Q[q].rays;
-					gq.count         = L.Q[q].count;
-					gq.looks         = looks;
-					gq.materialCount = looks.materialCount;
-					gq.lobes         = L.lobes;
-					if (!ctx->check(guideQueryQueue(ctx->guide, gq, n, on, ctx->smCount), "guide query kernel")) return KDN_CUDA_ERROR;
+				if (!last) {
+					HitArgs h;
+					h.world  = ctx->world;
+					h.rays   = L.Q[q].rays;
+					h.states = L.states;
+					h.n      = n;
+					h.hits   = L.hits;
+					h.count  = L.Q[q].count;
+					h.fetch  = L.fetch;
+					if (!ctx->check(launchHits(h, on, ctx->smCount), "hit kernel")) return KDN_CUDA_ERROR;
+					++launches;
+					if (guiding && round < kGuideDepth) {
+						GuideQueue gq;
+						gq.hits          = L.hits;
+						gq.rays          = L.Q[q].rays;
+						gq.count         = L.Q[q].count;
+						gq.looks         = looks;
+						gq.materialCount = looks.materialCount;
+						gq.lobes         = L.lobes;
+						if (!ctx->check(guideQueryQueue(ctx->guide, gq, n, on, ctx->smCount), "guide query kernel")) return KDN_CUDA_ERROR;
+						++launches;
+					}
+				}
+				if (round > 0) {
+					// the bounce before's lines that reached their lamps; lines still
+					// marching go on with the next round's
+					if (!ctx->check(launchLines(LP, L.S[q], L.S[nxt], lineCapacity, on, ctx->smCount), "lines kernel")) return KDN_CUDA_ERROR;
 					++launches;
 				}
+				if (last) continue;
+				ShadeArgs a;
+				a.paths         = LP;
+				a.in            = L.Q[q];
+				a.out           = L.Q[nxt];
+				a.shadow        = L.S[nxt];
+				a.hits          = L.hits;
+				a.states        = L.states;
+				a.looks         = looks;
+				a.capacity      = capacity;
+				a.lineCapacity  = lineCapacity;
+				a.error         = nullptr;
+				a.firstDistance = denoised ? static_cast<uint16_t*>(f.firstDistance.ptr) : nullptr;
+				a.firstNormal   = denoised ? static_cast<uint16_t*>(f.firstNormal.ptr) : nullptr;
+				a.firstAlbedo   = denoised ? static_cast<uint16_t*>(f.firstAlbedo.ptr) : nullptr;
+				a.firstLeaf     = denoised ? static_cast<uint32_t*>(f.firstLeaf.ptr) : nullptr;
+				a.lobes         = (guiding && round < kGuideDepth) ? L.lobes : nullptr;
+				a.guideShare    = ctx->guideShare;
+				a.records       = L.records;
+				if (!ctx->check(launchShade(c, a, on, ctx->smCount), "shade kernel")) return KDN_CUDA_ERROR;
+				++launches;
+				turn[l] = nxt;
 			}
-			if (!ctx->check(cudaMemsetAsync(L.S[nxt].count, 0, 4, on), "clear lines")) return KDN_CUDA_ERROR;
-			if (round > 0) {
-				// the bounce before's lines that reached their lamps; lines still
-				// marching go on with the next round's
-				if (!ctx->check(launchLines(LP, L.S[q], L.S[nxt], lineCapacity, on, ctx->smCount), "lines kernel")) return KDN_CUDA_ERROR;
+		}
+		for (int l = 0; l < members; ++l) {
+			const Lane& L        = lane[l];
+			const uint32_t first = (group + uint32_t(l)) * chunkPixels;
+			const uint32_t chunk = std::min(chunkPixels, pixels - first);
+			if (!ctx->check(launchFold(c, L.P, first, chunk, spp, static_cast<double*>(f.sums.ptr), denoised ? static_cast<float*>(f.frameLight.ptr) : nullptr, lanes[l], ctx->smCount), "fold kernel")) return KDN_CUDA_ERROR;
+			++launches;
+			if (training) {
+				if (!ctx->check(guideGather(ctx->guide, L.records, L.P.radiance, chunk * spp, uint64_t(pixels) * spp, uint32_t(fr->seed) * 0x85EBCA6Bu + first, lanes[l], ctx->smCount), "guide gather kernel")) return KDN_CUDA_ERROR;
 				++launches;
 			}
-			if (last) break;
-			if (!ctx->check(cudaMemsetAsync(L.Q[nxt].count, 0, 4, on), "clear queue")) return KDN_CUDA_ERROR;
-			ShadeArgs a;
-			a.paths         = LP;
-			a.in            = L.Q[q];
-			a.out           = L.Q[nxt];
-			a.shadow        = L.S[nxt];
-			a.hits          = L.hits;
-			a.states        = L.states;
-			a.looks         = looks;
-			a.capacity      = capacity;
-			a.lineCapacity  = lineCapacity;
-			a.error         = nullptr;
-			a.firstDistance = denoised ? static_cast<uint16_t*>(f.firstDistance.ptr) : nullptr;
-			a.firstNormal   = denoised ? static_cast<uint16_t*>(f.firstNormal.ptr) : nullptr;
-			a.firstAlbedo   = denoised ? static_cast<uint16_t*>(f.firstAlbedo.ptr) : nullptr;
-			a.firstLeaf     = denoised ? static_cast<uint32_t*>(f.firstLeaf.ptr) : nullptr;
-			a.lobes         = (guiding && round < kGuideDepth) ? L.lobes : nullptr;
-			a.guideShare    = ctx->guideShare;
-			a.records       = L.records;
-			if (!ctx->check(launchShade(c, a, on, ctx->smCount), "shade kernel")) return KDN_CUDA_ERROR;
-			++launches;
-			q = nxt;
-		}
-		if (!ctx->check(launchFold(c, LP, first, chunk, spp, static_cast<double*>(f.sums.ptr), denoised ? static_cast<float*>(f.frameLight.ptr) : nullptr, on, ctx->smCount), "fold kernel")) return KDN_CUDA_ERROR;
-		++launches;
-		if (training) {
-			if (!ctx->check(guideGather(ctx->guide, L.records, LP.radiance, n, uint64_t(pixels) * spp, uint32_t(fr->seed) * 0x85EBCA6Bu + first, on, ctx->smCount), "guide gather kernel")) return KDN_CUDA_ERROR;
-			++launches;
 		}
 	}
 	// the first lane goes on once the others and the surfaces pass are done

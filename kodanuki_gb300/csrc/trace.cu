@@ -181,11 +181,24 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 	const uint32_t n  = n1 + (args.secondCount ? *args.secondCount : 0u);
 	const unsigned lane = threadIdx.x & 31u;
 
-	if (args.left != nullptr && args.counters != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
-		const uint32_t left = *args.left;
-		if (left) atomicAdd(&args.counters[6], (unsigned long long) left);
+	if (blockIdx.x == 0 && threadIdx.x == 0) {
+		if (args.left != nullptr && args.counters != nullptr && *args.left) atomicAdd(&args.counters[6], (unsigned long long) *args.left);
+		for (uint32_t* c : { args.clear[0], args.clear[1] }) {
+			if (c != nullptr) *c = 0;
+		}
+		if (args.reached != nullptr) {
+			// the host's view of the frame: this launch has begun, and whether it has rays
+			if (n == 0) args.reached[1] = args.chunk;
+			__threadfence_system();
+			args.reached[0] = args.turn;
+		}
 	}
-	uint32_t mode = Fetch;
+	// a launch of few rays spreads them over its warps (a ray alone is marched
+	// soonest, and nothing else waits for the lanes)
+	const uint32_t warps = gridDim.x * (kTraceBlock / 32);
+	const uint32_t share = min(32u, (n + warps - 1u) / warps);
+	if (n == 0) return;
+	uint32_t mode = lane < share ? Fetch : Finished;
 	uint32_t ray  = 0;
 	float o[3] = { 0.0f, 0.0f, 0.0f }, d[3] = { 0.0f, 0.0f, 0.0f }, inv[3] = { 0.0f, 0.0f, 0.0f };
 	float t = 0.0f, up = 0.0f;
@@ -247,7 +260,7 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 		field.v[1] = 3.0e38f;
 		mode       = Evaluating;
 	};
-	uint32_t finished = 0; // lanes without a ray, the launch's all taken
+	uint32_t finished = 32u - share; // lanes without a ray, the launch's all taken
 
 	for (;;) {
 		const uint32_t modes      = __reduce_add_sync(0xFFFFFFFFu, mode);
@@ -533,6 +546,7 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 __global__ void __launch_bounds__(kTraceBlock) hitKernel(HitArgs args) {
 	const DeviceWorld& w = args.world;
 	const uint32_t n     = args.count ? *args.count : args.n;
+	if (args.fetch != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *args.fetch = 0;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 		const HitState h  = args.states[i];
 		const kdn_ray ray = args.rays[i];
@@ -625,10 +639,9 @@ cudaError_t launchTrace(const TraceArgs& args, cudaStream_t stream, int smCount)
 		resident = perSm;
 		sizedFor = shared;
 	}
-	const uint64_t wanted = (uint64_t(args.n) + kTraceBlock - 1) / kTraceBlock;
+	// a warp a ray where they are few: see the kernel's share
+	const uint64_t wanted = (uint64_t(args.n) + kTraceBlock / 32 - 1) / (kTraceBlock / 32);
 	const uint32_t blocks = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(wanted, uint64_t(smCount) * uint64_t(resident))));
-	cudaError_t e = cudaMemsetAsync(args.fetch, 0, sizeof(uint32_t), stream);
-	if (e != cudaSuccess) return e;
 	traceKernel<<<blocks, kTraceBlock, shared, stream>>>(args);
 	return cudaGetLastError();
 }
