@@ -29,7 +29,7 @@ def _compile(src: str, verbose: bool) -> str:
     obj = os.path.join(OUT, os.path.basename(src) + ".o")
     common = ["-O3", "-std=c++17", "-I", INCLUDE, "-I", CSRC, "-Xcompiler", "-fPIC,-ffp-contract=off", "--expt-relaxed-constexpr"]
     if src.endswith(".cu"):
-        # the denoiser keeps the reference's float order: no FMA contraction there
+        # the reconstruction members keep the reference's float order: no FMA but where it is written
         exact = ["-fmad=false"] if os.path.basename(src) in EXACT_FLOAT else []
         cmd = [NVCC] + ARCH + ["-lineinfo"] + common + exact + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj]
     else:

@@ -21,13 +21,13 @@ struct DenoiseArgs {
 	float* out;               // RGB a pixel
 	// scratch: guides and two light buffers
 	float4* guideA;           // x, y, z, plane offset
-	float4* guideB;           // normal, 1 / reach
-	float* sky;
+	float4* guideB;           // normal, 1 in the sky
+	float* near;              // 1 / (0.02 distance), 0 in the sky
 	float4* lightA;           // r, g, b, variance
 	float4* lightB;
 };
 
-// Bytes of scratch one pixel needs (guideA, guideB, sky, lightA, lightB).
+// Bytes of scratch one pixel needs (guideA, guideB, near, lightA, lightB).
 constexpr size_t kDenoiseScratchPerPixel = 16 + 16 + 4 + 16 + 16;
 
 cudaError_t launchDenoise(const DenoiseArgs& args, cudaStream_t stream);

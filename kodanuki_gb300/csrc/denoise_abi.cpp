@@ -38,7 +38,7 @@ kdn_status scratch(Context* ctx, size_t n, kdn::DenoiseArgs& a) {
 	a.guideB = a.guideA + n;
 	a.lightA = a.guideB + n;
 	a.lightB = a.lightA + n;
-	a.sky    = reinterpret_cast<float*>(a.lightB + n);
+	a.near   = reinterpret_cast<float*>(a.lightB + n);
 	return KDN_OK;
 }
 

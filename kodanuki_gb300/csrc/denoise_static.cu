@@ -99,7 +99,7 @@ kdn_status kdn_denoise_static(const kdn_denoise_frame* frame, const float* colou
 	a.guideB      = a.guideA + n;
 	a.lightA      = a.guideB + n;
 	a.lightB      = a.lightA + n;
-	a.sky         = reinterpret_cast<float*>(a.lightB + n);
+	a.near        = reinterpret_cast<float*>(a.lightB + n);
 	a.width       = frame->width;
 	a.height      = frame->height;
 	a.demodulated = frame->demodulated ? 1 : 0;

@@ -1098,7 +1098,7 @@ kdn_status renderFrame(Context* ctx, const kdn_frame* fr, float* out, cudaStream
 			if ((s = denoiseOnDevice(ctx, &df, ta.io.colour, ta.io.moment, ta.io.length, ta.io.centre_distance, ta.io.centre_normal, ta.io.centre_albedo,
 			                         ta.io.centre_leaf, drawnImage, stream)) != KDN_OK)
 				return s;
-			launches += 7;
+			launches += 6;
 		}
 		if (upsampled) {
 			// reconstruction/upsample as the chain's last member

@@ -356,6 +356,8 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 				const GpuLeaf leaf = w.leaves[cell.leaf];
 				MarchStep s;
 				memcpy(&s, leaf.params, sizeof s);
+				// from the first program on again, and counted again
+				for (uint32_t k = order >> 8 & 0xFFu; k-- > 0;) programSteps -= w.programs[leaf.first + k].marchSteps;
 				const bool one = leaf.count == 1 && s.op == FormPrimitive && leaf.marchCount == unitsOf(s);
 				const MarchParams c = paramsAt(w.march + leaf.march + 1);
 				MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
