@@ -358,9 +358,74 @@ struct TrainArgs {
 	uint32_t* error;
 };
 
-__global__ void __launch_bounds__(128, 1) trainKernel(const __grid_constant__ TrainArgs A) {
+// The training kernel's 512 threads are four groups of 128, a sample a row of
+// each: a group gathers and scatters four of the table's levels and works 16
+// columns of every layer's epilogue.
+constexpr uint32_t kTrainGroups = 4, kTrainThreads = 128 * kTrainGroups;
+// TMEM columns: two accumulators the forward pass alternates, the input
+// gradient, and the weight gradients, which a CTA sums over all of its tiles
+constexpr uint32_t kTmemDX = 128, kTmemDW = 192;
+
+// One 16-column slice of this thread's TMEM lane.
+__device__ __forceinline__ void tslice(uint32_t tmem, uint32_t col, float* v) { tload16(tmem + (((threadIdx.x >> 5) & 3u) * 32u << 16) + col, v); }
+
+// N columns from k0 on of row r of an image of K columns, and of column c of a
+// transposed image
+template <int K, int N>
+__device__ __forceinline__ void storePart(uint8_t* img, uint32_t r, uint32_t k0, const float* v, bool relu) {
+#pragma unroll
+	for (int k = 0; k < N; k += 8) {
+		uint32_t p[4];
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const float x = relu ? fmaxf(v[k + 2 * j], 0.0f) : v[k + 2 * j], y = relu ? fmaxf(v[k + 2 * j + 1], 0.0f) : v[k + 2 * j + 1];
+			__nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+			p[j]             = *reinterpret_cast<uint32_t*>(&h);
+		}
+		*reinterpret_cast<uint4*>(img + imgAt(r, k0 + k, K)) = make_uint4(p[0], p[1], p[2], p[3]);
+	}
+}
+template <int N>
+__device__ __forceinline__ void storeColumnPart(uint8_t* img, uint32_t c, uint32_t f0, const float* v) {
+#pragma unroll
+	for (int f = 0; f < N; ++f) *reinterpret_cast<__nv_bfloat16*>(img + imgAt(f0 + f, c, 128)) = __float2bfloat16_rn(v[f]);
+}
+template <int K, int N>
+__device__ __forceinline__ void readPart(const uint8_t* img, uint32_t r, uint32_t k0, float* v) {
+#pragma unroll
+	for (int k = 0; k < N; k += 8) {
+		const uint4 q       = *reinterpret_cast<const uint4*>(img + imgAt(r, k0 + k, K));
+		const uint32_t p[4] = { q.x, q.y, q.z, q.w };
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			__nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&p[j]);
+			v[k + 2 * j]     = __bfloat162float(h.x);
+			v[k + 2 * j + 1] = __bfloat162float(h.y);
+		}
+	}
+}
+
+// D += A . B^T over several instructions; first: the accumulator starts afresh
+__device__ __forceinline__ void mmaOnto(uint32_t d, uint32_t a, uint32_t b, uint32_t K, uint32_t N, bool first) {
+	const uint32_t idesc = idescOf(N);
+	for (uint32_t kk = 0; kk < K / 16u; ++kk) {
+		const uint64_t ad = descOf(a + kk * 256u, K);
+		const uint64_t bd = descOf(b + kk * 256u, K);
+		const uint32_t on = first ? kk : 1u;
+		asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(on) : "memory");
+	}
+}
+
+// A training step's gradients: a persistent CTA an SM takes tiles of 128
+// samples.  What bounds it is the table: 128 gathers and as many reductions of
+// two floats a sample, served by the L2; the rest is a chain of nine small
+// MMAs a tile.  With one thread a sample and one tile a CTA it took 277 us for
+// 65 536 samples: every thread went through its 16 levels' gathers one level
+// after the other and made 256 scalar reductions, and every tile added its
+// 14 336 weight gradients to the same addresses.
+__global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_constant__ TrainArgs A) {
 	extern __shared__ __align__(1024) uint8_t sm[];
-	const uint32_t tid = threadIdx.x;
+	const uint32_t tid = threadIdx.x, row = tid & 127u, group = tid >> 7;
 	uint8_t* X[4]      = { sm + kSX0, sm + kSX1, sm + kSX2, sm + kSX3 };
 	uint8_t* DY        = sm + kSDY;
 	uint8_t* DYT       = sm + kSDYT;
@@ -369,121 +434,160 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const __grid_constant__ Tr
 	uint32_t* slot     = reinterpret_cast<uint32_t*>(sm + kSBar + 16);
 	const uint32_t barLoad = sAddr(bars), barMma = sAddr(bars + 1);
 	if (tid == 0) initBarriers(barLoad, barMma);
-	if (tid < 32) allocTmem(sAddr(slot), 256);
+	if (tid < 32) allocTmem(sAddr(slot), 512);
 	// the padded rows of the transposed gradient stay zero
-	for (uint32_t i = tid; i < 32768u / 16u; i += 128u) reinterpret_cast<uint4*>(DYT)[i] = make_uint4(0, 0, 0, 0);
+	for (uint32_t i = tid; i < 32768u / 16u; i += kTrainThreads) reinterpret_cast<uint4*>(DYT)[i] = make_uint4(0, 0, 0, 0);
 	stage();
 	const uint32_t tmem = *slot;
 	if (tid == 0) loadImages(sAddr(sm), A.packed, kPacked, barLoad);
-
-	const uint32_t row = blockIdx.x * 128u + tid;
-	const bool live    = row < A.n;
-	float3 pos = make_float3(0, 0, 0), nrm = make_float3(0, 0, 0), dir = make_float3(0, 0, 1);
-	float weight = 0.0f;
-	float v[64];
-	if (live) {
-		const uint32_t s = uint32_t((uint64_t(A.first + row) * A.stride + A.offset) % A.total);
-		const float* r   = A.samples + size_t(s) * kGuideSampleFloats;
-		pos              = make_float3(r[0], r[1], r[2]);
-		nrm              = make_float3(r[3], r[4], r[5]);
-		dir              = make_float3(r[6], r[7], r[8]);
-		weight           = r[9];
-		encodeRow(A.table, A.tableLog2, A.region, pos, nrm, v);
-	} else {
-#pragma unroll
-		for (int k = 0; k < int(kIn); ++k) v[k] = 0.0f;
-	}
-	storeRow<48>(X[0], tid, v, false);
-	bool ok = waitBar(barLoad, 0);
-	stage();
+	bool loaded    = false, failed = false;
 	uint32_t phase = 0;
-	bool failed    = __syncthreads_or(!ok);
-	// forward: layer l into TMEM columns 64 l
+	float lossSum  = 0.0f;
+	const uint32_t tiles = (A.n + 127u) / 128u;
+	for (uint32_t tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
+		const bool first    = tile == blockIdx.x;
+		const uint32_t at   = tile * 128u + row;
+		const bool live     = at < A.n;
+		const float* sample = A.samples + size_t(live ? uint32_t((uint64_t(A.first + at) * A.stride + A.offset) % A.total) : 0u) * kGuideSampleFloats;
+		// the input: each group its four levels' eight features; the last the
+		// normal, 1 and zeros besides
+		float u[3] = { 0.0f, 0.0f, 0.0f };
+		float v[16];
+		if (live) unitOf(A.region, make_float3(sample[0], sample[1], sample[2]), u);
 #pragma unroll
-	for (int l = 0; l < 4; ++l) {
-		if (failed) break;
-		if (tid == 0) {
-			mma(tmem + 64u * l, sAddr(X[l]), sAddr(sm + imgW(l)), nIn(l), nOut(l));
-			commit(barMma);
+		for (int k = 0; k < 4; ++k) {
+			float a = 0.0f, b = 0.0f;
+			if (live) {
+				const int l = int(group) * 4 + k;
+				uint32_t idx[8];
+				float w[8];
+				cornersAt(u, l, A.tableLog2, idx, w);
+				const __half2* level = A.table + (size_t(l) << A.tableLog2);
+#pragma unroll
+				for (int c = 0; c < 8; ++c) {
+					const float2 f = __half22float2(__ldg(level + idx[c]));
+					a              = __fadd_rn(a, __fmul_rn(w[c], f.x));
+					b              = __fadd_rn(b, __fmul_rn(w[c], f.y));
+				}
+			}
+			v[2 * k]     = a;
+			v[2 * k + 1] = b;
 		}
-		ok = waitBar(barMma, phase);
-		phase ^= 1u;
-		if ((failed = __syncthreads_or(!ok))) break;
-		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-		if (l < 3) {
-			tload<64>(tmem, 64u * l, v);
-			storeRow<64>(X[l + 1], tid, v, true);
+		storePart<48, 8>(X[0], row, group * 8u, v, false);
+		if (group == 3) {
+#pragma unroll
+			for (int k = 0; k < 16; ++k) v[k] = 0.0f;
+			if (live) v[0] = sample[3], v[1] = sample[4], v[2] = sample[5], v[3] = 1.0f;
+			storePart<48, 16>(X[0], row, 32u, v, false);
+		}
+		bool ok = loaded || waitBar(barLoad, 0);
+		loaded  = true;
+		stage();
+		failed = __syncthreads_or(!ok);
+		// forward: layer l into TMEM columns 64 (l & 1)
+#pragma unroll
+		for (int l = 0; l < 4; ++l) {
+			if (failed) break;
+			if (tid == 0) {
+				mma(tmem + 64u * (l & 1), sAddr(X[l]), sAddr(sm + imgW(l)), nIn(l), nOut(l));
+				commit(barMma);
+			}
+			ok = waitBar(barMma, phase);
+			phase ^= 1u;
+			if ((failed = __syncthreads_or(!ok))) break;
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			if (l < 3) {
+				tslice(tmem, 64u * (l & 1) + group * 16u, v);
+				storePart<64, 16>(X[l + 1], row, group * 16u, v, true);
+				stage();
+			}
+		}
+		if (!failed) {
+			// the loss of a row wants all of its outputs in one thread
+			if (group == 0) {
+				float o[48], g[48];
+				tload<48>(tmem, 64u, o);
+				float rowLoss = 0.0f;
+				if (live) lossRow(o, make_float3(sample[6], sample[7], sample[8]), sample[9], 1.0f / float(A.n), g, rowLoss);
+				else {
+#pragma unroll
+					for (int k = 0; k < 48; ++k) g[k] = 0.0f;
+				}
+				storeRow<48>(DY, row, g, false);
+				storeColumn<48>(DYT, row, g);
+				lossSum += rowLoss;
+			}
+			stage();
+		}
+		// backward: layer l's input gradient, and its weight gradient onto the CTA's
+#pragma unroll
+		for (int l = 3; l >= 0; --l) {
+			if (failed) break;
+			const uint32_t k0 = group * 16u;
+			float xr[16];
+			if (k0 < nIn(l)) {
+				if (l == 0) readPart<48, 16>(X[0], row, k0, xr);
+				else readPart<64, 16>(X[l], row, k0, xr);
+				storeColumnPart<16>(XT, row, k0, xr);
+			}
+			stage();
+			if (tid == 0) {
+				mma(tmem + kTmemDX, sAddr(DY), sAddr(sm + imgWt(l)), nOut(l), nIn(l));
+				mmaOnto(tmem + kTmemDW + 64u * l, sAddr(DYT), sAddr(XT), 128u, nIn(l), first);
+				commit(barMma);
+			}
+			ok = waitBar(barMma, phase);
+			phase ^= 1u;
+			if ((failed = __syncthreads_or(!ok))) break;
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			if (l > 0) {
+				tslice(tmem, kTmemDX + k0, v);
+#pragma unroll
+				for (int k = 0; k < 16; ++k) v[k] = xr[k] > 0.0f ? v[k] : 0.0f;
+				storePart<64, 16>(DY, row, k0, v, false);
+				storeColumnPart<16>(DYT, row, k0, v);
+			} else {
+				tslice(tmem, kTmemDX + (group >> 1) * 16u, v);
+				if (live) {
+#pragma unroll
+					for (int k = 0; k < 4; ++k) {
+						const int lv = int(group) * 4 + k;
+						uint32_t idx[8];
+						float w[8];
+						cornersAt(u, lv, A.tableLog2, idx, w);
+						float* level  = A.tGrad + (size_t(lv) << A.tableLog2) * 2u;
+						const float a = group & 1u ? v[8 + 2 * k] : v[2 * k], b = group & 1u ? v[9 + 2 * k] : v[2 * k + 1];
+#pragma unroll
+						for (int c = 0; c < 8; ++c)
+							asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(level + 2u * idx[c]), "f"(w[c] * a), "f"(w[c] * b) : "memory");
+					}
+				}
+			}
 			stage();
 		}
 	}
-	float g[64];
-	if (!failed) {
-		tload<48>(tmem, 192u, v);
-		float rowLoss = 0.0f;
-		if (live) lossRow(v, dir, weight, 1.0f / float(A.n), g, rowLoss);
-		else {
+	// the CTA's weight gradients and loss
+	if (!failed && blockIdx.x < tiles) {
 #pragma unroll
-			for (int k = 0; k < 48; ++k) g[k] = 0.0f;
-		}
-		storeRow<48>(DY, tid, g, false);
-		storeColumn<48>(DYT, tid, g);
-		for (int o = 16; o > 0; o >>= 1) rowLoss += __shfl_xor_sync(0xFFFFFFFFu, rowLoss, o);
-		if ((tid & 31u) == 0 && rowLoss != 0.0f) atomicAdd(A.loss, rowLoss / float(A.n));
-		stage();
-	}
-	// backward: layer l's input gradient into columns 0.., its weight gradient into 64..
+		for (int l = 0; l < 4; ++l) {
+			const uint32_t k0 = group * 16u;
+			if (k0 >= nIn(l)) continue;
+			float v[16];
+			tslice(tmem, kTmemDW + 64u * l + k0, v);
+			if (row < nOut(l)) {
+				float* dw = A.wGrad + wOff(l) + row * nIn(l) + k0;
 #pragma unroll
-	for (int l = 3; l >= 0; --l) {
-		if (failed) break;
-		float xr[64];
-		if (l == 0) readRow<48>(X[0], tid, xr);
-		else readRow<64>(X[l], tid, xr);
-		if (l == 0) storeColumn<48>(XT, tid, xr);
-		else storeColumn<64>(XT, tid, xr);
-		stage();
-		if (tid == 0) {
-			mma(tmem, sAddr(DY), sAddr(sm + imgWt(l)), nOut(l), nIn(l));
-			mma(tmem + 64u, sAddr(DYT), sAddr(XT), 128u, nIn(l));
-			commit(barMma);
-		}
-		ok = waitBar(barMma, phase);
-		phase ^= 1u;
-		if ((failed = __syncthreads_or(!ok))) break;
-		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-		if (l == 0) tload<48>(tmem, 64u, v);
-		else tload<64>(tmem, 64u, v);
-		if (tid < nOut(l)) {
-			float* dw = A.wGrad + wOff(l) + tid * nIn(l);
-			for (uint32_t k = 0; k < nIn(l); ++k)
-				if (v[k] != 0.0f) atomicAdd(dw + k, v[k]);
-		}
-		if (l == 0) tload<48>(tmem, 0u, v);
-		else tload<64>(tmem, 0u, v);
-		if (l > 0) {
-#pragma unroll
-			for (int k = 0; k < 64; ++k) g[k] = xr[k] > 0.0f ? v[k] : 0.0f;
-			storeRow<64>(DY, tid, g, false);
-			storeColumn<64>(DYT, tid, g);
-		} else if (live) {
-			float u[3];
-			unitOf(A.region, pos, u);
-			for (int lv = 0; lv < int(kLevels); ++lv) {
-				uint32_t idx[8];
-				float w[8];
-				cornersAt(u, lv, A.tableLog2, idx, w);
-				float* level = A.tGrad + (size_t(lv) << A.tableLog2) * 2u;
-#pragma unroll
-				for (int c = 0; c < 8; ++c) {
-					atomicAdd(level + 2u * idx[c], w[c] * v[2 * lv]);
-					atomicAdd(level + 2u * idx[c] + 1u, w[c] * v[2 * lv + 1]);
-				}
+				for (int k = 0; k < 16; k += 4)
+					asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dw + k), "f"(v[k]), "f"(v[k + 1]), "f"(v[k + 2]), "f"(v[k + 3]) : "memory");
 			}
 		}
-		stage();
+		for (int o = 16; o > 0; o >>= 1) lossSum += __shfl_xor_sync(0xFFFFFFFFu, lossSum, o);
+		if ((tid & 31u) == 0 && lossSum != 0.0f) atomicAdd(A.loss, lossSum / float(A.n));
 	}
 	if (failed && tid == 0) atomicExch(A.error, 1u);
+	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
-	if (tid < 32) freeTmem(tmem, 256);
+	if (tid < 32) freeTmem(tmem, 512);
 }
 
 struct QueryArgs {
@@ -701,12 +805,12 @@ TrainArgs trainArgs(kdn_guide* g) {
 	return a;
 }
 
-cudaError_t launchTrain(const TrainArgs& a, cudaStream_t s) {
+cudaError_t launchTrain(const TrainArgs& a, cudaStream_t s, int smCount) {
 	static std::once_flag once;
 	static cudaError_t setup = cudaSuccess;
 	std::call_once(once, [] { setup = cudaFuncSetAttribute(trainKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTrainSmem)); });
 	if (setup != cudaSuccess) return setup;
-	trainKernel<<<(a.n + 127u) / 128u, 128, kTrainSmem, s>>>(a);
+	trainKernel<<<std::min((a.n + 127u) / 128u, uint32_t(std::max(1, smCount))), kTrainThreads, kTrainSmem, s>>>(a);
 	return cudaGetLastError();
 }
 
@@ -742,7 +846,7 @@ kdn_status trainOver(kdn_guide* g, uint32_t total, uint32_t batch, uint32_t step
 		a.first  = uint32_t((uint64_t(k) * batch) % total);
 		a.n      = std::min(batch, total);
 		a.offset = 0;
-		GCHECK(launchTrain(a, s), "guide train kernel");
+		GCHECK(launchTrain(a, s, g->smCount), "guide train kernel");
 		GCHECK(adamStep(g, s), "guide adam");
 	}
 	return KDN_OK;
@@ -932,7 +1036,7 @@ kdn_status kdn_guide_gradients(kdn_guide* g, const float* samples, uint32_t n, f
 	a.first     = 0;
 	a.n         = n;
 	a.total     = n;
-	GCHECK(launchTrain(a, g->stream), "guide train kernel");
+	GCHECK(launchTrain(a, g->stream, g->smCount), "guide train kernel");
 	GCHECK(cudaStreamSynchronize(g->stream), "guide train kernel");
 	if ((s = checkError(g)) != KDN_OK) return s;
 	if (loss) GCHECK(cudaMemcpy(loss, g->loss, 4, cudaMemcpyDeviceToHost), "guide loss");
@@ -960,7 +1064,7 @@ kdn_status kdn_guide_train(kdn_guide* g, const float* samples, uint32_t n, uint3
 	a.total     = n;
 	a.first     = uint32_t((uint64_t(steps - 1) * batch) % n);
 	a.n         = std::min(batch, n);
-	GCHECK(launchTrain(a, g->stream), "guide train kernel");
+	GCHECK(launchTrain(a, g->stream, g->smCount), "guide train kernel");
 	GCHECK(adamStep(g, g->stream), "guide adam");
 	GCHECK(cudaStreamSynchronize(g->stream), "guide train");
 	if ((s = checkError(g)) != KDN_OK) return s;
