@@ -2,9 +2,9 @@
 // in single precision.
 //
 //  - evalSlots: the march's form.  Values live in register slots held in
-//    shared memory, one column per thread: slot s of thread t is at
-//    slots[s * blockDim.x + t], so a warp's accesses to one slot hit 32
-//    consecutive banks.
+//    shared memory, a column each for the rays of a block: slot s of ray r is at
+//    slots[s * stride + r], so a warp's accesses to one slot hit the banks of
+//    its rays' places.
 //  - evalDual:  the value and gradient (forward mode, sdf/numbers.cpp:440
 //    Dual) over the same slots, 4 floats a slot.
 //  - evalSsa:   every step's value kept by step number, for the walk back from
@@ -212,7 +212,7 @@ KDN_HD MarchParams paramsAt(const MarchStep* unit) {
 }
 
 // One step of the march form (world.h MarchStep) at a point but a primitive,
-// over a thread's slots: r = post(form, w); a rare step runs the reference
+// over a ray's slots: r = post(form, w); a rare step runs the reference
 // operation.  Writes the result to its slot and returns it.
 KDN_HD float marchStep(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride) {
 	slots[SlotImm * stride] = s.value;
@@ -261,8 +261,8 @@ KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float
 	return r;
 }
 
-// One program at one point; slots is this thread's column base (stride
-// blockDim.x), with the constants set.  Returns the program's value, which
+// One program at one point; slots is its ray's column (stride the
+// block's rays), with the constants set.  Returns the program's value, which
 // its last step makes.
 KDN_HD float evalSlots(const MarchStep* __restrict__ code, uint32_t count, float* slots, uint32_t stride, const float p[3]) {
 	setPoint(slots, stride, p);

@@ -19,13 +19,19 @@ namespace kdn {
 namespace {
 
 constexpr int kTraceBlock = 128;
-// A thread's register slots are a column of shared memory, one float a slot.
-constexpr uint32_t kStride = kTraceBlock;
-// rays of a warp that may wait at their ends before the warp sees to them
-constexpr uint32_t kWaiting = 8;
-// steps a ray takes in a shaped cell (world.h LeafShape), and program steps,
-// a turn (2 to 8 and 1 to 4 measured within 3%); with kFew rays in hand, kAlone
-constexpr uint32_t kMovesPerTurn = 4, kStepsPerTurn = 2;
+// Rays a warp holds.  With one a lane, 12 of 32 lanes work in a turn; with 64
+// in hand 20 to 24 do (config 2's full frame 480 ms against 425 ms, a launch
+// of 960 x 540 x 8 of its rays 3.57 against 2.80 ms).  48: 460 ms; 96 take
+// the L1 the programs are read through: 480 ms.
+constexpr uint32_t kPool = 64;
+// A ray's register slots are a column of shared memory, one float a slot.
+constexpr uint32_t kStride = kTraceBlock / 32 * kPool;
+// rays of a warp that may wait at their ends before the warp sees to them (16
+// and 32 measured within 2%)
+constexpr uint32_t kWaiting = 24;
+// steps a ray takes in a shaped cell (world.h LeafShape) a turn (1 to 8
+// measured within 3%); with kFew rays in hand, kAlone
+constexpr uint32_t kMovesPerTurn = 4;
 constexpr uint32_t kFew = 4, kAlone = 64;
 // steps worked out at once where a ray is seen to stay in its cell
 constexpr uint32_t kRun = 8;
@@ -154,24 +160,46 @@ __device__ __noinline__ InsideStop insideStop(const DeviceWorld& w, const uint32
 	return InsideStop { 0, 0, 0, steps };
 }
 
-// The march as a step machine.  Each thread holds one ray at a time.  A ray
-// waits to be located, or to step in a cell whose field its leaf record holds
-// (empty, or a single slab or sphere: a few operations in registers), or for
-// the programs of its cell, a step of theirs at a time; every turn the warp
-// does the one thing most of its rays wait for.  Rays that have landed or
-// ended wait until there are several, and the ended take the next rays of the
-// launch (one atomic a warp).
+// The march as a step machine.  A warp holds a pool of rays, more than it has
+// lanes, in shared memory.  A ray waits to be located, or to step in a cell
+// whose field its leaf record holds (empty, or a single slab or sphere: a few
+// operations in registers), or for the programs of its cell, a step of theirs
+// at a time; every turn the warp does the one thing most of its rays wait for,
+// a lane a ray of those.  Rays that have landed or ended wait until there are
+// several, and the ended take the next rays of the launch (one atomic a warp).
 // A mode's number is its count's place in the warp's sum of them.
 enum LaneMode : uint32_t { Locating = 1, Stepping = 1 << 8, Evaluating = 1 << 16, Fetch = 1 << 24, Landed = 3 << 24, Finished = 5 << 24 };
 
-// Five blocks an SM (96 registers) hold the machine's state in registers: six
-// spill it (config 2's frame 550 against 489 ms), four hide less of the
-// loads' latency (492 against 475 ms).
-__global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_constant__ TraceArgs args) {
-	extern __shared__ float slotMemory[];
+constexpr uint32_t kOwn = (kPool + 31) / 32; // rays of the pool whose modes a lane counts
+constexpr uint32_t kWarps = kTraceBlock / 32;
+
+// A warp's pool: each row a float4 or less of every ray.
+struct Pool {
+	float4 origin[kPool];    // o, up
+	float4 direction[kPool]; // d, stepLimit | within << 31
+	float4 inverse[kPool];   // 1 / d, the ray's index in the launch
+	float4 at[kPool];        // t, step, the cell's exit and leaf
+	float4 wall[kPool];      // the cell's walls; its shape and, from bit 8, what a step in it adds to the program step count
+	// the field of a slab or a sphere.  In a cell of programs: what the ones
+	// evaluated so far came to, the least value and the second least (from
+	// inside a solid, the least magnitude), the last step's value, and pc
+	float4 field[kPool];
+	uint2 program[kPool];    // where the program in hand ends; which it is, of how many, and which was least (a byte each)
+	uint32_t mode[kPool];
+	uint32_t taken[32];      // the rays of this turn
+};
+
+// Four blocks an SM: 111 registers, 28 KB of shared memory and the slots'
+// columns a block.  Five leave less L1 (config 2's full frame 453 against 431 ms).
+// What bounds it: the issue of instructions while the SMs are full (51% of the
+// cycles, at 17 of 32 lanes), and in a launch by itself the last rays of it
+// (the SMs stand idle for 40% of 2.80 ms).
+__global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_constant__ TraceArgs args) {
+	extern __shared__ float4 poolMemory[];
 	const DeviceWorld& w = args.world;
-	float* slots         = slotMemory + threadIdx.x;
-	setConstants(slots, kStride);
+	Pool& pool           = reinterpret_cast<Pool*>(poolMemory)[threadIdx.x / 32];
+	// a ray's register slots: a column each
+	float* const columns = reinterpret_cast<float*>(reinterpret_cast<Pool*>(poolMemory) + kWarps) + threadIdx.x / 32 * kPool;
 	// capped rays in the low 16 bits, carried ones in the high: one register
 	uint32_t marchSteps = 0, programSteps = 0, traced = 0, cappedCarried = 0, longest = 0;
 	// the steps a ray may take in this launch: a launch's budget, or the cap
@@ -195,32 +223,28 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 	}
 	// a launch of few rays spreads them over its warps (a ray alone is marched
 	// soonest, and nothing else waits for the lanes)
-	const uint32_t warps = gridDim.x * (kTraceBlock / 32);
-	const uint32_t share = min(32u, (n + warps - 1u) / warps);
+	const uint32_t warps = gridDim.x * kWarps;
+	const uint32_t share = min(kPool, (n + warps - 1u) / warps);
 	if (n == 0) return;
-	uint32_t mode = lane < share ? Fetch : Finished;
-	uint32_t ray  = 0;
-	float o[3] = { 0.0f, 0.0f, 0.0f }, d[3] = { 0.0f, 0.0f, 0.0f }, inv[3] = { 0.0f, 0.0f, 0.0f };
+	for (uint32_t r = lane; r < kPool; r += 32u) {
+		pool.mode[r] = r < share ? Fetch : Finished;
+		setConstants(columns + r, kStride);
+	}
+	__syncwarp();
+
+	// the ray in a lane's hands this turn
+	uint32_t r    = 0, mode = 0;
+	float o[3] = { 0.0f, 0.0f, 0.0f }, d[3] = { 0.0f, 0.0f, 0.0f };
 	float t = 0.0f, up = 0.0f;
 	bool within   = false; // the ray started inside a solid
 	uint32_t step = 0;
 	// where the ray's march stops in this launch: the cap, or sooner its budget
 	uint32_t stepLimit = 0;
-	// the ray's cell, its shape, and what a step in it adds to the program step count
-	uint32_t shape = 0, cost = 0;
+	uint32_t kind      = 0; // shape and cost
 	Ahead cell { kNoLeaf, { 0.0f, 0.0f, 0.0f }, 0.0f };
-	// the field of a slab or a sphere; in a cell of programs, what the ones
-	// evaluated so far came to: v[0] the least value, v[1] the second least
-	// (from inside a solid, the least magnitude)
-	MarchParams field { { 0.0f, 0.0f, 0.0f, 0.0f } };
-	// the program in hand: its code from pc to end, its last step's value, and
-	// which it is, of how many, and which was least (a byte each)
-	uint32_t pc = 0, end = 0, order = 0;
-	float last = 0.0f;
-	MarchStep next {};
 	// a ray ends: its state, the step counts, and the next ray
 	auto done = [&](HitState h) {
-		args.states[ray] = h;
+		args.states[__float_as_uint(pool.inverse[r].w)] = h;
 		marchSteps += h.steps; // less the steps it had when taken (at the fetch)
 		longest = max(longest, h.steps);
 		cappedCarried += h.kind == kCarried ? 0x10000u : (h.steps >= args.maxSteps ? 1u : 0u);
@@ -235,7 +259,6 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 		done(HitState { carried ? kCarried : 0u, t, kNoLeaf, 0, step });
 		return true;
 	};
-
 	// a ray goes on from t to on, its march step taken: to the end of its march,
 	// on in its cell, or out of it.  A step too small to move it would be taken
 	// again to the limit: cost, what one adds to the program step count.
@@ -249,43 +272,75 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 		const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
 		mode             = inside(cell.wall, p, d) ? Stepping : Locating;
 	};
-	// a ray starts on the programs of its cell
-	auto start = [&](const GpuLeaf& leaf) {
-		pc    = leaf.march;
-		end   = leaf.march + leaf.marchCount;
-		order = leaf.count;
-		cost  = leaf.marchSteps;
-		memcpy(&next, leaf.params, sizeof next);
-		field.v[0] = 3.0e38f;
-		field.v[1] = 3.0e38f;
-		mode       = Evaluating;
+	// the ray of a turn, from the pool and back
+	auto load = [&]() {
+		const float4 a = pool.origin[r], b = pool.direction[r], c = pool.at[r], e = pool.wall[r];
+		o[0] = a.x, o[1] = a.y, o[2] = a.z, up = a.w;
+		d[0] = b.x, d[1] = b.y, d[2] = b.z;
+		stepLimit    = __float_as_uint(b.w) & 0x7FFFFFFFu;
+		within       = __float_as_uint(b.w) >> 31 != 0u;
+		t            = c.x;
+		step         = __float_as_uint(c.y);
+		cell.exit    = c.z;
+		cell.leaf    = __float_as_uint(c.w);
+		cell.wall[0] = e.x, cell.wall[1] = e.y, cell.wall[2] = e.z;
+		kind         = __float_as_uint(e.w);
 	};
-	uint32_t finished = 32u - share; // lanes without a ray, the launch's all taken
+	auto keep = [&]() {
+		pool.at[r]   = make_float4(t, __uint_as_float(step), cell.exit, __uint_as_float(cell.leaf));
+		pool.mode[r] = mode;
+	};
+	// the rays in one mode, a lane each: how many (the others take none)
+	uint32_t own[kOwn];
+	auto modeAt = [&](uint32_t k) { return kPool % 32 == 0 || lane + k * 32u < kPool ? pool.mode[lane + k * 32u] : 0u; };
+	auto take = [&](uint32_t which) {
+		uint32_t first = 0;
+		const unsigned before = (1u << lane) - 1u;
+		for (uint32_t k = 0; k < kOwn; ++k) {
+			const unsigned those = __ballot_sync(0xFFFFFFFFu, own[k] == which);
+			const uint32_t place = first + uint32_t(__popc(those & before));
+			if (own[k] == which && place < 32u) pool.taken[place] = lane + k * 32u;
+			first += uint32_t(__popc(those));
+		}
+		__syncwarp();
+		r = pool.taken[lane];
+		return min(first, 32u);
+	};
+	uint32_t finished = kPool - share; // places without a ray, the launch's all taken
 
 	for (;;) {
-		const uint32_t modes      = __reduce_add_sync(0xFFFFFFFFu, mode);
+		uint32_t sum = 0;
+		for (uint32_t k = 0; k < kOwn; ++k) {
+			own[k] = modeAt(k);
+			sum += own[k];
+		}
+		const uint32_t modes      = __reduce_add_sync(0xFFFFFFFFu, sum);
 		const uint32_t locating   = modes & 0xFFu, stepping = modes >> 8 & 0xFFu, evaluating = modes >> 16 & 0xFFu;
 		const uint32_t busy       = locating + stepping + evaluating;
-		const uint32_t waiting    = 32u - busy - finished;
+		const uint32_t waiting    = kPool - busy - finished;
 		if (waiting >= kWaiting || waiting > busy) {
-			if (mode == Landed) {
+			if (lane < take(Landed)) {
+				load();
+				mode = Landed;
 				// field and order hold what the march step came to: the least of the
 				// cell's programs, the second least (from inside, the least magnitude)
 				// and the least's index
 				const GpuLeaf leaf = w.leaves[cell.leaf];
+				const float4 field = pool.field[r];
+				float* slots       = columns + r;
 				const float p[3]   = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-				const Field f { field.v[0], order >> 16, leaf.count, leaf.first };
+				const Field f { field.x, pool.program[r].y >> 16, leaf.count, leaf.first };
 				const float3 at = make_float3(p[0], p[1], p[2]), along = make_float3(d[0], d[1], d[2]);
 				if (!within) {
 					const float big = fmaxf(fabsf(p[0]), fmaxf(fabsf(p[1]), fabsf(p[2])));
-					const bool tied = field.v[1] - field.v[0] <= 2e-6f * (1.0f + big);
+					const bool tied = field.y - field.x <= 2e-6f * (1.0f + big);
 					const uint32_t winner = tied ? winnerAt(w, at, along, f, slots) : f.index;
 					done(HitState { 1, t, f.first, winner, step });
 				} else {
 					// sphereFromInside: stand on the nearest surface and read the field past it
 					const float inset = 2.0f * tolerance(p), past = t + inset;
-					const InsideStop stop = insideStop(w, args.objectMaterial, args.rays[ray].within, at, make_float3(o[0] + d[0] * past, o[1] + d[1] * past, o[2] + d[2] * past),
-					                                   along, f, slots);
+					const InsideStop stop = insideStop(w, args.objectMaterial, args.rays[__float_as_uint(pool.inverse[r].w)].within, at,
+					                                   make_float3(o[0] + d[0] * past, o[1] + d[1] * past, o[2] + d[2] * past), along, f, slots);
 					programSteps += stop.steps;
 					if (stop.kind == 0) {
 						uint32_t each = stop.steps;
@@ -298,29 +353,32 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 						done(HitState { stop.kind, t, stop.first, stop.index, step });
 					}
 				}
+				keep();
 			}
+			__syncwarp();
+			for (uint32_t k = 0; k < kOwn; ++k) own[k] = modeAt(k);
 			// take new rays, one atomic a warp
-			const unsigned mask = __ballot_sync(0xFFFFFFFFu, mode == Fetch);
-			if (mask) {
+			const uint32_t wanted = take(Fetch);
+			if (wanted) {
 				uint32_t base = 0;
-				const int leader = __ffs(mask) - 1;
-				if (int(lane) == leader) base = atomicAdd(args.fetch, uint32_t(__popc(mask)));
-				base = __shfl_sync(0xFFFFFFFFu, base, leader);
-				if (mode == Fetch) {
-					ray = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
+				if (lane == 0) base = atomicAdd(args.fetch, wanted);
+				base = __shfl_sync(0xFFFFFFFFu, base, 0);
+				if (lane < wanted) {
+					uint32_t ray = base + lane;
 					if (ray >= n) {
-						mode = Finished;
+						pool.mode[r] = Finished;
 					} else {
 						if (ray >= n1) ray = args.second + (ray - n1);
-						const kdn_ray r = args.rays[ray];
-						within          = r.inside != 0;
+						const kdn_ray from = args.rays[ray];
+						within             = from.inside != 0;
+						float inv[3];
 						for (int a = 0; a < 3; ++a) {
-							o[a]   = r.origin[a];
-							d[a]   = r.direction[a];
+							o[a]   = from.origin[a];
+							d[a]   = from.direction[a];
 							inv[a] = slopeOf(d[a]);
 						}
 						float lo = 0.0f;
-						up       = r.far;
+						up       = from.far;
 						for (int a = 0; a < 3; ++a) {
 							const float x = (w.lower[a] - o[a]) * inv[a];
 							const float y = (w.lower[a] + w.size[a] - o[a]) * inv[a];
@@ -330,7 +388,7 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 						t    = lo;
 						step = 0;
 						// a carried ray goes on where its march stood
-						if (args.carry != nullptr && (r.pad_[0] & kRayResumes)) {
+						if (args.carry != nullptr && (from.pad_[0] & kRayResumes)) {
 							const uint2 c = args.carry[ray];
 							t             = __uint_as_float(c.x);
 							step          = c.y;
@@ -339,117 +397,146 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 						}
 						stepLimit = min(args.maxSteps, step + allowance);
 						marchSteps -= step;
+						pool.origin[r]    = make_float4(o[0], o[1], o[2], up);
+						pool.direction[r] = make_float4(d[0], d[1], d[2], __uint_as_float(stepLimit | (within ? 0x80000000u : 0u)));
+						pool.inverse[r]   = make_float4(inv[0], inv[1], inv[2], __uint_as_float(ray));
 						if (up < lo) done(HitState { 0, t, kNoLeaf, 0, step });
 						else if (!over()) mode = Locating;
+						keep();
 					}
 				}
+				__syncwarp();
 			}
-			finished = __popc(__ballot_sync(0xFFFFFFFFu, mode == Finished));
-			if (finished == 32) break;
+			finished = 0;
+			for (uint32_t k = 0; k < kOwn; ++k) finished += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, modeAt(k) == Finished)));
+			if (finished == kPool) break;
 			continue;
 		}
 		if (evaluating >= locating && evaluating >= stepping) {
-			if (mode == Evaluating && busy <= kFew) {
-				// few rays in hand: whole march steps at a time, each as soon as the
-				// one before is done (a ray that skims a box takes thousands; the
-				// turns above cost one 480 ns a step, these 200)
-				const GpuLeaf leaf = w.leaves[cell.leaf];
-				MarchStep s;
-				memcpy(&s, leaf.params, sizeof s);
-				// from the first program on again, and counted again
-				for (uint32_t k = order >> 8 & 0xFFu; k-- > 0;) programSteps -= w.programs[leaf.first + k].marchSteps;
-				const bool one = leaf.count == 1 && s.op == FormPrimitive && leaf.marchCount == unitsOf(s);
-				const MarchParams c = paramsAt(w.march + leaf.march + 1);
-				MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
-				if (one && s.m & PrimSized) h = paramsAt(w.march + leaf.march + 2);
-				uint32_t turns = kAlone;
+			if (lane < take(Evaluating)) {
+				load();
+				mode          = Evaluating;
+				float4 f      = pool.field[r];
+				uint2 program = pool.program[r];
+				float* slots  = columns + r;
+				float last    = f.z;
+				// the program in hand: its code from pc to end, its last step's value, and
+				// which it is, of how many, and which was least (a byte each)
+				uint32_t pc = __float_as_uint(f.w), end = program.x, order = program.y, cost = kind >> 8;
+				if (busy <= kFew) {
+					// few rays in hand: whole march steps at a time, each as soon as the
+					// one before is done (a ray that skims a box takes thousands; the
+					// turns below cost one 480 ns a step, these 250)
+					const GpuLeaf leaf = w.leaves[cell.leaf];
+					MarchStep s;
+					memcpy(&s, leaf.params, sizeof s);
+					// from the first program on again, and counted again
+					for (uint32_t k = order >> 8 & 0xFFu; k-- > 0;) programSteps -= w.programs[leaf.first + k].marchSteps;
+					const bool one = leaf.count == 1 && s.op == FormPrimitive && leaf.marchCount == unitsOf(s);
+					const MarchParams c = paramsAt(w.march + leaf.march + 1);
+					MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
+					if (one && s.m & PrimSized) h = paramsAt(w.march + leaf.march + 2);
+					uint32_t turns = kAlone;
 #pragma unroll 1
-				do {
-					const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-					float least = 3.0e38f, second = 3.0e38f;
-					uint32_t index = 0, each = 0;
-					if (one) {
-						least = primitiveValue(s, c, h, p[0], p[1], p[2]);
-						each  = leaf.marchSteps;
-						if (within) second = fabsf(least);
-					} else {
+					do {
+						const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+						float least = 3.0e38f, second = 3.0e38f;
+						uint32_t index = 0, each = 0;
+						if (one) {
+							least = primitiveValue(s, c, h, p[0], p[1], p[2]);
+							each  = leaf.marchSteps;
+							if (within) second = fabsf(least);
+						} else {
 #pragma unroll 1
-						for (uint32_t k = 0; k < leaf.count; ++k) {
-							const GpuProgram g = w.programs[leaf.first + k];
-							const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
-							const bool lesser  = v < least;
-							each += g.marchSteps;
-							second = within ? fminf(second, fabsf(v)) : lesser ? least : fminf(second, v);
-							least  = lesser ? v : least;
-							index  = lesser ? k : index;
+							for (uint32_t k = 0; k < leaf.count; ++k) {
+								const GpuProgram g = w.programs[leaf.first + k];
+								const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
+								const bool lesser  = v < least;
+								each += g.marchSteps;
+								second = within ? fminf(second, fabsf(v)) : lesser ? least : fminf(second, v);
+								least  = lesser ? v : least;
+								index  = lesser ? k : index;
+							}
 						}
+						programSteps += each;
+						++step;
+						const float go = within ? second : least;
+						if (go < tolerance(p)) {
+							f.x   = least;
+							f.y   = second;
+							order = index << 16;
+							mode  = Landed;
+							break;
+						}
+						goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), each);
+					} while (mode == Stepping && --turns != 0u);
+					if (mode == Stepping) {
+						pc    = leaf.march;
+						end   = leaf.march + leaf.marchCount;
+						order = leaf.count;
+						cost  = leaf.marchSteps;
+						f.x = f.y = 3.0e38f;
+						mode  = Evaluating;
 					}
-					programSteps += each;
-					++step;
-					const float go = within ? second : least;
-					if (go < tolerance(p)) {
-						field.v[0] = least;
-						field.v[1] = second;
-						order      = index << 16;
-						mode       = Landed;
-						break;
-					}
-					goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), each);
-				} while (mode == Stepping && --turns != 0u);
-				if (mode == Stepping) start(leaf);
-			} else if (mode == Evaluating) {
-				// the next step's code is loaded a step ahead
-				float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-				uint32_t turns = kStepsPerTurn;
-#pragma unroll 1
-				do {
-					const MarchStep s     = next;
+				} else {
+					const float p[3]      = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+					const MarchStep s     = w.march[pc];
 					const MarchStep* unit = w.march + pc + 1;
 					pc += unitsOf(s);
-					if (pc < end) next = w.march[pc];
 					if (primitiveStep(s)) {
 						last = primitiveStepValue(s, unit, slots, kStride, p[0], p[1], p[2], last);
 					} else {
 						setPoint(slots, kStride, p);
 						last = marchStep(s, unit, slots, kStride);
 					}
-					if (pc != end) continue;
-					programSteps += cost;
-					uint32_t k        = order >> 8 & 0xFFu;
-					const bool lesser = last < field.v[0];
-					field.v[1]        = within ? fminf(field.v[1], fabsf(last)) : lesser ? field.v[0] : fminf(field.v[1], last);
-					field.v[0]        = lesser ? last : field.v[0];
-					if (lesser) order = (order & 0x0000FFFFu) | k << 16;
-					if (++k < (order & 0xFFu)) {
-						const GpuProgram g = w.programs[w.leaves[cell.leaf].first + k];
-						pc    = g.march;
-						end   = g.march + g.marchCount;
-						order = (order & 0x00FF00FFu) | k << 8;
-						cost  = g.marchSteps;
-						next  = w.march[pc];
-						continue;
+					if (pc == end) {
+						programSteps += cost;
+						uint32_t k         = order >> 8 & 0xFFu;
+						const bool lesser  = last < f.x;
+						f.y                = within ? fminf(f.y, fabsf(last)) : lesser ? f.x : fminf(f.y, last);
+						f.x                = lesser ? last : f.x;
+						const GpuLeaf leaf = w.leaves[cell.leaf];
+						if (lesser) order = (order & 0x0000FFFFu) | k << 16;
+						if (++k < (order & 0xFFu)) {
+							const GpuProgram g = w.programs[leaf.first + k];
+							pc    = g.march;
+							end   = g.march + g.marchCount;
+							order = (order & 0x00FF00FFu) | k << 8;
+							cost  = g.marchSteps;
+						} else {
+							// stop on the surface or go on by the value
+							const float go = within ? f.y : f.x;
+							++step;
+							if (go < tolerance(p)) {
+								mode = Landed;
+							} else {
+								const float on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
+								uint32_t each  = 0;
+								if (on == t) {
+									for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
+								}
+								goOn(on, each);
+								pc    = leaf.march;
+								end   = leaf.march + leaf.marchCount;
+								order = leaf.count;
+								cost  = leaf.marchSteps;
+								f.x = f.y = 3.0e38f;
+								if (mode == Stepping) mode = Evaluating;
+							}
+						}
 					}
-					// stop on the surface or go on by the value
-					const float go = within ? field.v[1] : field.v[0];
-					++step;
-					if (go < tolerance(p)) {
-						mode = Landed;
-						break;
-					}
-					const GpuLeaf leaf = w.leaves[cell.leaf];
-					const float on     = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
-					uint32_t each      = 0;
-					if (on == t) {
-						for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
-					}
-					goOn(on, each);
-					if (mode != Stepping) break;
-					start(leaf);
-					for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
-				} while (--turns != 0u);
+				}
+				keep();
+				pool.wall[r].w  = __uint_as_float((kind & 0xFFu) | cost << 8);
+				pool.field[r]   = make_float4(f.x, f.y, last, __uint_as_float(pc));
+				pool.program[r] = make_uint2(end, order);
 			}
 		} else if (locating >= stepping) {
-			if (mode == Locating) {
+			if (lane < take(Locating)) {
+				load();
+				mode             = Locating;
+				const float4 i   = pool.inverse[r];
+				const float inv[3] = { i.x, i.y, i.z };
 				// the cell of the point; an empty one is left at once
 				const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
 				int place[3];
@@ -472,14 +559,24 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 					over();
 				} else {
 					const GpuLeaf leaf = w.leaves[cell.leaf];
-					shape              = leaf.shape;
-					cost               = leaf.marchSteps;
-					for (int a = 0; a < 4; ++a) field.v[a] = leaf.params[a];
-					mode = Stepping;
-					if (shape == ShapePrograms) start(leaf);
+					mode               = Stepping;
+					if (leaf.shape == ShapePrograms) {
+						mode            = Evaluating;
+						pool.field[r]   = make_float4(3.0e38f, 3.0e38f, 0.0f, __uint_as_float(leaf.march));
+						pool.program[r] = make_uint2(leaf.march + leaf.marchCount, leaf.count);
+					} else {
+						pool.field[r] = make_float4(leaf.params[0], leaf.params[1], leaf.params[2], leaf.params[3]);
+					}
+					pool.wall[r] = make_float4(cell.wall[0], cell.wall[1], cell.wall[2], __uint_as_float(leaf.shape | uint32_t(leaf.marchSteps) << 8));
 				}
+				keep();
 			}
-		} else if (mode == Stepping) {
+		} else if (lane < take(Stepping)) {
+			load();
+			mode = Stepping;
+			const float4 kept = pool.field[r];
+			const MarchParams field { { kept.x, kept.y, kept.z, kept.w } };
+			const uint32_t shape = kind & 0xFFu, cost = kind >> 8;
 			// a ray that skims the ground takes tens of thousands of these steps,
 			// alone in its warp, each waiting on the one before
 			uint32_t turns      = busy <= kFew ? kAlone : kMovesPerTurn;
@@ -515,15 +612,16 @@ __global__ void __launch_bounds__(kTraceBlock, 5) traceKernel(const __grid_const
 				programSteps += cost;
 				++step;
 				if (go < tol) { // it lands: the one program's value, its own second
-					field.v[0] = value;
-					field.v[1] = within ? go : 3.0e38f;
-					order      = 0;
-					mode       = Landed;
+					pool.field[r]     = make_float4(value, within ? go : 3.0e38f, 0.0f, 0.0f);
+					pool.program[r].y = 0u;
+					mode              = Landed;
 					break;
 				}
 				goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), cost);
 			} while (mode == Stepping && --turns != 0u);
+			keep();
 		}
+		__syncwarp();
 	}
 	if (args.counters) {
 		// one add per warp
@@ -628,10 +726,10 @@ __global__ void __launch_bounds__(kTraceBlock) hitKernel(HitArgs args) {
 
 cudaError_t launchTrace(const TraceArgs& args, cudaStream_t stream, int smCount) {
 	if (args.n == 0) return cudaSuccess;
-	// a thread's register slots in shared memory, as many as the world's
+	// the warps' pools and a ray's register slots, as many as the world's
 	// largest march program uses: the rest of the SM's shared memory stays
 	// L1 for the programs' code
-	const size_t shared = size_t(std::max<uint32_t>(1, std::min(args.world.marchSlots, kMaxSlots))) * kTraceBlock * sizeof(float);
+	const size_t shared = sizeof(Pool) * kWarps + size_t(std::max<uint32_t>(kMarchFirstSlot, std::min(args.world.marchSlots, kMaxSlots))) * kStride * sizeof(float);
 	// persistent blocks: as many as fit on the SMs at once, fewer for a small launch
 	static thread_local size_t sizedFor = 0;
 	static thread_local int resident    = 0;
@@ -656,7 +754,7 @@ cudaError_t launchHits(const HitArgs& args, cudaStream_t stream, int smCount) {
 }
 
 cudaError_t setTraceAttributes() {
-	return cudaFuncSetAttribute(traceKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxSlots * kTraceBlock * sizeof(float)));
+	return cudaFuncSetAttribute(traceKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(Pool) * kWarps + kMaxSlots * kStride * sizeof(float)));
 }
 
 } // namespace kdn
