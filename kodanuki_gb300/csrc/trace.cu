@@ -30,9 +30,11 @@ constexpr uint32_t kStride = kTraceBlock / 32 * kPool;
 // and 32 measured within 2%)
 constexpr uint32_t kWaiting = 24;
 // steps a ray takes in a shaped cell (world.h LeafShape) a turn (1 to 8
-// measured within 3%); with kFew rays in hand, kAlone
+// measured within 3%)
 constexpr uint32_t kMovesPerTurn = 4;
-constexpr uint32_t kFew = 4, kAlone = 64;
+// with kFew rays in hand or less (2, 4, 8, 16: a 256 x 256 frame of 16 samples
+// 14.0, 10.1, 9.4, 9.3 ms), a ray takes up to kAlone steps a turn
+constexpr uint32_t kFew = 8, kAlone = 256;
 // steps worked out at once where a ray is seen to stay in its cell
 constexpr uint32_t kRun = 8;
 
@@ -97,6 +99,71 @@ __device__ __noinline__ Ahead deepCell(const DeviceWorld& w, float3 point, int32
 	return c;
 }
 
+// A program at a point, out of line: the turns' code below is what the
+// instruction cache is for (config 2's full frame 400 ms, 430 with it inline).
+__device__ __noinline__ float programValue(const MarchStep* code, uint32_t count, float* slots, float3 at) {
+	const float p[3] = { at.x, at.y, at.z };
+	return evalSlots(code, count, slots, kStride, p);
+}
+
+// A primitive step along one ray, with what does not change from a point to
+// the next worked out: the ray's part along each term's axis, and the choices
+// as masks.  The value is primitiveValue's to the bit but for a zero's sign (a
+// value of zero lands, and is worked out again), for a ray of finite parts.
+struct AlongRay {
+	float from[3], by[3];   // the point's coordinate: from + by * t
+	float c[3], h[3];       // the slabs
+	float low[3];           // 0 where the term is squared by its positive part
+	uint32_t keep[3], turn[3], has[3]; // |u|, -u and a term left out, as masks
+	float r, e;
+	uint32_t within;        // the inside term's mask
+	bool fused1, fused2, single, plain, third;
+};
+
+__device__ __forceinline__ AlongRay alongRay(const MarchStep& s, const MarchParams& c, const MarchParams& h, const float o[3], const float d[3]) {
+	AlongRay a;
+	const uint32_t terms[3] = { s.a, s.b, s.c };
+	for (uint32_t k = 0; k < 3; ++k) {
+		const uint32_t axis = terms[k] & 3u, side = terms[k] >> kTermSideShift;
+		a.from[k] = axis == 0 ? o[0] : axis == 1 ? o[1] : o[2];
+		a.by[k]   = axis == 0 ? d[0] : axis == 1 ? d[1] : d[2];
+		a.c[k]    = -c.v[k];
+		a.h[k]    = -h.v[k];
+		a.low[k]  = s.flags & SumPositive0 << k ? 0.0f : -__int_as_float(0x7F800000);
+		a.keep[k] = side == SideAbs ? 0x7FFFFFFFu : 0xFFFFFFFFu;
+		a.turn[k] = side == SideNegative ? 0x80000000u : 0u;
+		a.has[k]  = s.flags & SumHas0 << k ? 0xFFFFFFFFu : 0u;
+	}
+	a.r      = h.v[3];
+	a.e      = -c.v[3];
+	a.within = s.m & PrimInside ? 0xFFFFFFFFu : 0u;
+	a.fused1 = s.flags & SumFused1;
+	a.fused2 = s.flags & SumFused2;
+	a.single = s.m & PrimSingle;
+	a.plain  = s.m & PrimPlain;
+	a.third  = s.m & PrimThird;
+	return a;
+}
+
+__device__ __forceinline__ float masked(float x, uint32_t mask) { return __uint_as_float(__float_as_uint(x) & mask); }
+
+__device__ __forceinline__ float valueAlong(const AlongRay& a, float t) {
+	float u[3], p[3];
+	for (int k = 0; k < 3; ++k) {
+		const float x = __fadd_rn(fmaf(a.by[k], t, a.from[k]), a.c[k]);
+		u[k]          = __fadd_rn(__fadd_rn(__uint_as_float((__float_as_uint(x) & a.keep[k]) ^ a.turn[k]), a.h[k]), a.r);
+		p[k]          = masked(fmaxf(u[k], a.low[k]), a.has[k]);
+	}
+	float sum = __fmul_rn(p[0], p[0]);
+	sum       = a.fused1 ? fmaf(p[1], p[1], sum) : __fadd_rn(__fmul_rn(p[1], p[1]), sum);
+	sum       = a.fused2 ? fmaf(p[2], p[2], sum) : __fadd_rn(__fmul_rn(p[2], p[2]), sum);
+	float f   = marchSqrt(sum);
+	f         = a.single ? fmaxf(p[0] + p[1] + p[2], 0.0f) : f; // one term, the others zero
+	f         = a.plain ? u[0] : f;
+	f         = __fadd_rn(f, masked(fminf(fmaxf(u[0], fmaxf(u[1], a.third ? u[2] : u[1])), 0.0f), a.within));
+	return __fadd_rn(f, a.e);
+}
+
 struct Field {
 	float least;    // least program value
 	uint32_t index; // which kept program is least
@@ -110,7 +177,7 @@ __device__ __forceinline__ Field fieldAt(const DeviceWorld& w, const float p[3],
 	Field f { 3.0e38f, 0, leaf.shape == ShapeEmpty ? 0u : leaf.count, leaf.first };
 	for (uint32_t k = 0; k < f.count; ++k) {
 		const GpuProgram g = w.programs[f.first + k];
-		const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
+		const float v      = programValue(w.march + g.march, g.marchCount, slots, make_float3(p[0], p[1], p[2]));
 		steps += g.marchSteps;
 		if (v < f.least) {
 			f.least = v;
@@ -131,8 +198,8 @@ __device__ __noinline__ uint32_t winnerAt(const DeviceWorld& w, float3 at, float
 	float onWinner   = 3.0e38f;
 	for (uint32_t k = 0; k < f.count; ++k) {
 		const GpuProgram g = w.programs[f.first + k];
-		if (!(evalSlots(w.march + g.march, g.marchCount, slots, kStride, p) - f.least <= band)) continue;
-		const float on = evalSlots(w.march + g.march, g.marchCount, slots, kStride, q);
+		if (!(programValue(w.march + g.march, g.marchCount, slots, make_float3(p[0], p[1], p[2])) - f.least <= band)) continue;
+		const float on = programValue(w.march + g.march, g.marchCount, slots, make_float3(q[0], q[1], q[2]));
 		if (on < onWinner) {
 			onWinner = on;
 			winner   = k;
@@ -413,7 +480,146 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 			continue;
 		}
 		if (evaluating >= locating && evaluating >= stepping) {
-			if (lane < take(Evaluating)) {
+			const uint32_t count = take(Evaluating);
+			if (busy <= kFew) {
+				// few rays in hand: whole march steps at a time, a share of the lanes a
+				// ray (a ray that skims a box takes thousands of steps, and nothing else
+				// is left to wait for).  Where the cell's programs are primitives, each
+				// joined to the one before, a lane works out one primitive from
+				// registers; else a program, or every so many.  A step is bound by its
+				// chain of instructions, some 300 ns of them; a lane a ray took 500 for
+				// a primitive and 1400 for a program of three (a 256 x 256 frame of 16
+				// samples 13.3 against 9.4 ms, the interactive one of 4096 primitives
+				// 18 against 14, the preview 5.1 against 3.4).
+				const uint32_t wide  = count == 1u ? 32u : count == 2u ? 16u : count <= 4u ? 8u : 4u; // lanes a ray
+				const uint32_t place = lane / wide, mine = lane & (wide - 1u);
+				const bool leads     = mine == 0u && place < count;
+				r                    = pool.taken[place < count ? place : 0u];
+				load();
+				const GpuLeaf leaf = w.leaves[cell.leaf];
+				// the lane's primitive; which of its program's it is, and if the last
+				MarchStep s {};
+				uint32_t unit = 0, total = 0, nth = 0, longestProgram = 0, each = 0;
+				bool ends = false, plain = true;
+#pragma unroll 1
+				for (uint32_t k = 0; k < leaf.count; ++k) {
+					uint32_t pc = leaf.march, end = leaf.march + leaf.marchCount, cost = leaf.marchSteps;
+					if (k != 0u) {
+						const GpuProgram g = w.programs[leaf.first + k];
+						pc   = g.march;
+						end  = g.march + g.marchCount;
+						cost = g.marchSteps;
+					}
+					each += cost;
+					uint32_t at = 0;
+#pragma unroll 1
+					while (plain && pc < end) {
+						const MarchStep x   = w.march[pc];
+						const uint32_t next = pc + unitsOf(x);
+						plain = primitiveStep(x) && total < wide && (x.op == FormPrimitive || x.m & PrimPrevious || x.w == SlotImm);
+						if (total == mine) {
+							s    = x;
+							unit = pc;
+							nth  = at;
+							ends = next == end;
+						}
+						++total;
+						++at;
+						pc = next;
+					}
+					longestProgram = max(longestProgram, at);
+				}
+				for (int a = 0; a < 3; ++a) plain = plain && fabsf(o[a]) < 3.0e38f && fabsf(d[a]) < 3.0e38f;
+				plain = __all_sync(0xFFFFFFFFu, plain);
+				MarchParams c { { 0.0f, 0.0f, 0.0f, 0.0f } }, h { { 0.0f, 0.0f, 0.0f, -0.0f } };
+				const bool holds = plain && mine < total; // a lane with a primitive
+				if (holds) c = paramsAt(w.march + unit + 1);
+				if (holds && s.m & PrimSized) h = paramsAt(w.march + unit + 2);
+				const AlongRay primitive = alongRay(s, c, h, o, d);
+				const uint32_t post = s.op & kMarchPostMask;
+				const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, longestProgram), most = __reduce_max_sync(0xFFFFFFFFu, plain ? total : wide);
+				// the programs begin again at the first, and are counted again
+				if (leads) {
+					for (uint32_t k = pool.program[r].y >> 8 & 0xFFu; k-- > 0;) programSteps -= w.programs[leaf.first + k].marchSteps;
+				}
+				float* slots   = columns + lane; // no ray is within a program now
+				float p[3]     = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				uint32_t taken = 0;
+				// a ray's march: on in its cell, landed, ended, or out of the cell
+				enum { On, Lands, Ends, Leaves } state = On;
+#pragma unroll 1
+				for (uint32_t turn = 1; turn <= kAlone; ++turn) {
+					float v = 3.0e38f;
+					if (plain) {
+						const float f = valueAlong(primitive, t);
+						float last    = nth == 0u && post != PostNone ? posted(post, f, s.value, s.value, s.quarter) : f;
+#pragma unroll 1
+						for (uint32_t k = 1; k < rounds; ++k) {
+							const float prior = __shfl_up_sync(0xFFFFFFFFu, last, 1);
+							if (nth == k && post != PostNone) last = posted(post, f, s.m & PrimPrevious ? prior : s.value, s.value, s.quarter);
+						}
+						if (holds && ends) v = fminf(3.0e38f, within ? fabsf(last) : last);
+					} else {
+#pragma unroll 1
+						for (uint32_t q = mine; q < leaf.count; q += wide) {
+							const GpuProgram g = w.programs[leaf.first + q];
+							const float u      = programValue(w.march + g.march, g.marchCount, slots, make_float3(p[0], p[1], p[2]));
+							v                  = fminf(v, within ? fabsf(u) : u);
+						}
+					}
+					// the least of a ray's lanes (of those that hold any)
+					for (uint32_t k = 1; k < most; k *= 2u) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, int(k)));
+					v = __shfl_sync(0xFFFFFFFFu, v, 0, int(wide));
+					if (state == On) {
+						const float on = fminf(t + v, fmaxf(cell.exit, t) + nudge(t));
+						++step;
+						++taken;
+						if (v < tolerance(p)) {
+							state = Lands;
+						} else {
+							if (on == t) {
+								taken += stepLimit - step;
+								step = stepLimit;
+							}
+							t = on;
+							for (int a = 0; a < 3; ++a) p[a] = o[a] + d[a] * t;
+							state = !(step < stepLimit && t <= up) ? Ends : inside(cell.wall, p, d) ? On : Leaves;
+						}
+					}
+					// until all have done with their cells, and where one has, for some steps
+					const unsigned on = __ballot_sync(0xFFFFFFFFu, state == On);
+					if (on == 0u || (on != 0xFFFFFFFFu && turn >= kRun)) break;
+				}
+				if (leads) {
+					programSteps += taken * each;
+					pool.program[r] = make_uint2(leaf.march + leaf.marchCount, leaf.count);
+					float4 field    = make_float4(3.0e38f, 3.0e38f, 0.0f, __uint_as_float(leaf.march));
+					mode            = Evaluating;
+					if (state == Lands) {
+						// the least of the programs, the second (from inside, the least
+						// magnitude) and the least's index
+						uint32_t index = 0;
+#pragma unroll 1
+						for (uint32_t k = 0; k < leaf.count; ++k) {
+							const GpuProgram g = w.programs[leaf.first + k];
+							const float v      = programValue(w.march + g.march, g.marchCount, slots, make_float3(p[0], p[1], p[2]));
+							const bool lesser  = v < field.x;
+							field.y            = within ? fminf(field.y, fabsf(v)) : lesser ? field.x : fminf(field.y, v);
+							field.x            = lesser ? v : field.x;
+							index              = lesser ? k : index;
+						}
+						pool.program[r].y = index << 16;
+						mode              = Landed;
+					} else if (state == Leaves) {
+						mode = Locating;
+					} else {
+						over();
+					}
+					keep();
+					pool.field[r]  = field;
+					pool.wall[r].w = __uint_as_float((kind & 0xFFu) | uint32_t(leaf.marchSteps) << 8);
+				}
+			} else if (lane < count) {
 				load();
 				mode          = Evaluating;
 				float4 f      = pool.field[r];
@@ -423,106 +629,49 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 				// the program in hand: its code from pc to end, its last step's value, and
 				// which it is, of how many, and which was least (a byte each)
 				uint32_t pc = __float_as_uint(f.w), end = program.x, order = program.y, cost = kind >> 8;
-				if (busy <= kFew) {
-					// few rays in hand: whole march steps at a time, each as soon as the
-					// one before is done (a ray that skims a box takes thousands; the
-					// turns below cost one 480 ns a step, these 250)
-					const GpuLeaf leaf = w.leaves[cell.leaf];
-					MarchStep s;
-					memcpy(&s, leaf.params, sizeof s);
-					// from the first program on again, and counted again
-					for (uint32_t k = order >> 8 & 0xFFu; k-- > 0;) programSteps -= w.programs[leaf.first + k].marchSteps;
-					const bool one = leaf.count == 1 && s.op == FormPrimitive && leaf.marchCount == unitsOf(s);
-					const MarchParams c = paramsAt(w.march + leaf.march + 1);
-					MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
-					if (one && s.m & PrimSized) h = paramsAt(w.march + leaf.march + 2);
-					uint32_t turns = kAlone;
-#pragma unroll 1
-					do {
-						const float p[3] = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-						float least = 3.0e38f, second = 3.0e38f;
-						uint32_t index = 0, each = 0;
-						if (one) {
-							least = primitiveValue(s, c, h, p[0], p[1], p[2]);
-							each  = leaf.marchSteps;
-							if (within) second = fabsf(least);
-						} else {
-#pragma unroll 1
-							for (uint32_t k = 0; k < leaf.count; ++k) {
-								const GpuProgram g = w.programs[leaf.first + k];
-								const float v      = evalSlots(w.march + g.march, g.marchCount, slots, kStride, p);
-								const bool lesser  = v < least;
-								each += g.marchSteps;
-								second = within ? fminf(second, fabsf(v)) : lesser ? least : fminf(second, v);
-								least  = lesser ? v : least;
-								index  = lesser ? k : index;
-							}
-						}
-						programSteps += each;
-						++step;
-						const float go = within ? second : least;
-						if (go < tolerance(p)) {
-							f.x   = least;
-							f.y   = second;
-							order = index << 16;
-							mode  = Landed;
-							break;
-						}
-						goOn(fminf(t + go, fmaxf(cell.exit, t) + nudge(t)), each);
-					} while (mode == Stepping && --turns != 0u);
-					if (mode == Stepping) {
-						pc    = leaf.march;
-						end   = leaf.march + leaf.marchCount;
-						order = leaf.count;
-						cost  = leaf.marchSteps;
-						f.x = f.y = 3.0e38f;
-						mode  = Evaluating;
-					}
+				const float p[3]      = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
+				const MarchStep s     = w.march[pc];
+				const MarchStep* unit = w.march + pc + 1;
+				pc += unitsOf(s);
+				if (primitiveStep(s)) {
+					last = primitiveStepValue(s, unit, slots, kStride, p[0], p[1], p[2], last);
 				} else {
-					const float p[3]      = { o[0] + d[0] * t, o[1] + d[1] * t, o[2] + d[2] * t };
-					const MarchStep s     = w.march[pc];
-					const MarchStep* unit = w.march + pc + 1;
-					pc += unitsOf(s);
-					if (primitiveStep(s)) {
-						last = primitiveStepValue(s, unit, slots, kStride, p[0], p[1], p[2], last);
+					setPoint(slots, kStride, p);
+					last = marchStep(s, unit, slots, kStride);
+				}
+				if (pc == end) {
+					programSteps += cost;
+					uint32_t k         = order >> 8 & 0xFFu;
+					const bool lesser  = last < f.x;
+					f.y                = within ? fminf(f.y, fabsf(last)) : lesser ? f.x : fminf(f.y, last);
+					f.x                = lesser ? last : f.x;
+					const GpuLeaf leaf = w.leaves[cell.leaf];
+					if (lesser) order = (order & 0x0000FFFFu) | k << 16;
+					if (++k < (order & 0xFFu)) {
+						const GpuProgram g = w.programs[leaf.first + k];
+						pc    = g.march;
+						end   = g.march + g.marchCount;
+						order = (order & 0x00FF00FFu) | k << 8;
+						cost  = g.marchSteps;
 					} else {
-						setPoint(slots, kStride, p);
-						last = marchStep(s, unit, slots, kStride);
-					}
-					if (pc == end) {
-						programSteps += cost;
-						uint32_t k         = order >> 8 & 0xFFu;
-						const bool lesser  = last < f.x;
-						f.y                = within ? fminf(f.y, fabsf(last)) : lesser ? f.x : fminf(f.y, last);
-						f.x                = lesser ? last : f.x;
-						const GpuLeaf leaf = w.leaves[cell.leaf];
-						if (lesser) order = (order & 0x0000FFFFu) | k << 16;
-						if (++k < (order & 0xFFu)) {
-							const GpuProgram g = w.programs[leaf.first + k];
-							pc    = g.march;
-							end   = g.march + g.marchCount;
-							order = (order & 0x00FF00FFu) | k << 8;
-							cost  = g.marchSteps;
+						// stop on the surface or go on by the value
+						const float go = within ? f.y : f.x;
+						++step;
+						if (go < tolerance(p)) {
+							mode = Landed;
 						} else {
-							// stop on the surface or go on by the value
-							const float go = within ? f.y : f.x;
-							++step;
-							if (go < tolerance(p)) {
-								mode = Landed;
-							} else {
-								const float on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
-								uint32_t each  = 0;
-								if (on == t) {
-									for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
-								}
-								goOn(on, each);
-								pc    = leaf.march;
-								end   = leaf.march + leaf.marchCount;
-								order = leaf.count;
-								cost  = leaf.marchSteps;
-								f.x = f.y = 3.0e38f;
-								if (mode == Stepping) mode = Evaluating;
+							const float on = fminf(t + go, fmaxf(cell.exit, t) + nudge(t));
+							uint32_t each  = 0;
+							if (on == t) {
+								for (uint32_t k = 0; k < leaf.count; ++k) each += w.programs[leaf.first + k].marchSteps;
 							}
+							goOn(on, each);
+							pc    = leaf.march;
+							end   = leaf.march + leaf.marchCount;
+							order = leaf.count;
+							cost  = leaf.marchSteps;
+							f.x = f.y = 3.0e38f;
+							if (mode == Stepping) mode = Evaluating;
 						}
 					}
 				}
