@@ -6,9 +6,10 @@
 //    slots[s * stride + r], so a warp's accesses to one slot hit the banks of
 //    its rays' places.
 //  - evalDual:  the value and gradient (forward mode, sdf/numbers.cpp:440
-//    Dual) over the same slots, 4 floats a slot.
-//  - evalSsa:   every step's value kept by step number, for the walk back from
-//    the result that names the source leaf (sdf/program.cpp:478).
+//    Dual) over the same slots, 4 floats a slot, and every step's value kept
+//    by step number.
+//  - sourceOf:  the walk back from the result that names the source leaf
+//    (sdf/program.cpp:478).
 #pragma once
 
 #include "world.h"
@@ -328,12 +329,53 @@ __device__ __forceinline__ DualF dualStep(uint8_t op, DualF a, DualF b, DualF c,
 	}
 }
 
-__device__ __forceinline__ DualF evalDual(const GpuStep* __restrict__ code, uint32_t count, uint32_t resultSlot, DualF* slots, const float p[3]) {
+// A step of the operations that distances are made of, worked out together and
+// the step's picked, so the lanes of a warp at different steps do not split;
+// dualStep's to the bit.  A gradient is fa * x.g, and + fb * b.g for a sum or a
+// product, x being an operand or a coordinate's own.
+__device__ __forceinline__ DualF commonDual(uint8_t op, DualF a, DualF b, float value, const float p[3]) {
+	const bool lesser = a.v <= b.v, greater = a.v >= b.v, negative = a.v < 0.0f;
+	const bool second = op == OpMin ? !lesser : op == OpMax && !greater;
+	const bool sum = op == OpAdd || op == OpSubtract, product = op == OpMultiply, point = op >= OpPointX && op <= OpPointZ;
+	const bool turns = op == OpNegate || (op == OpAbs && negative);
+	const float m    = fmaxf(a.v, 0.0f);
+	DualF x;
+	x.v  = second ? b.v : op == OpConstant ? value : op == OpPointX ? p[0] : op == OpPointY ? p[1] : op == OpPointZ ? p[2] : a.v;
+	x.g0 = point ? (op == OpPointX ? 1.0f : 0.0f) : op == OpConstant ? 0.0f : second ? b.g0 : a.g0;
+	x.g1 = point ? (op == OpPointY ? 1.0f : 0.0f) : op == OpConstant ? 0.0f : second ? b.g1 : a.g1;
+	x.g2 = point ? (op == OpPointZ ? 1.0f : 0.0f) : op == OpConstant ? 0.0f : second ? b.g2 : a.g2;
+	const float fa = product ? b.v : op == OpPosSq ? 2.0f * m : turns ? -1.0f : 1.0f;
+	const float fb = product ? a.v : op == OpSubtract ? -1.0f : 1.0f;
+	const bool two = sum || product;
+	DualF r;
+	r.v  = op == OpAdd ? a.v + b.v : op == OpSubtract ? a.v - b.v : product ? a.v * b.v : op == OpPosSq ? m * m : turns ? -a.v : x.v;
+	r.g0 = two ? fa * x.g0 + fb * b.g0 : fa * x.g0;
+	r.g1 = two ? fa * x.g1 + fb * b.g1 : fa * x.g1;
+	r.g2 = two ? fa * x.g2 + fb * b.g2 : fa * x.g2;
+	return r;
+}
+
+__device__ __forceinline__ bool isCommon(uint8_t op) {
+	constexpr uint64_t those = 1ull << OpConstant | 1ull << OpPointX | 1ull << OpPointY | 1ull << OpPointZ | 1ull << OpAdd | 1ull << OpSubtract | 1ull << OpMultiply | 1ull << OpNegate | 1ull << OpAbs | 1ull << OpMin | 1ull << OpMax | 1ull << OpPosSq;
+	return op < 64 && those >> op & 1u;
+}
+
+// The value and gradient, and every step's value by step number in v (for
+// sourceOf), but where one is not a number: then false, and v is to be made.
+__device__ __forceinline__ bool evalDual(const GpuStep* __restrict__ code, uint32_t count, uint32_t resultSlot, DualF* slots, float* v, const float p[3], DualF& result) {
+	bool numbers = true;
 	for (uint32_t i = 0; i < count; ++i) {
 		const GpuStep s = code[i];
-		slots[s.dst]    = dualStep(s.op, slots[s.a], slots[s.b], slots[s.c], s.value, p);
+		const DualF a = slots[s.a], b = slots[s.b];
+		DualF r;
+		if (isCommon(s.op)) r = commonDual(s.op, a, b, s.value, p);
+		else r = dualStep(s.op, a, b, slots[s.c], s.value, p);
+		slots[s.dst] = r;
+		v[i]         = r.v;
+		numbers      = numbers && r.v == r.v;
 	}
-	return slots[resultSlot];
+	result = slots[resultSlot];
+	return numbers;
 }
 
 __device__ __forceinline__ bool isJoin(uint8_t op) { return op == OpMin || op == OpSmin || op == OpMax || op == OpNegate || op == OpSelect; }
@@ -348,11 +390,11 @@ __device__ __forceinline__ uint32_t chosenOperand(uint8_t op, const SsaOps& o, c
 	}
 }
 
-// Every step's value by step number, then the walk back through the joins
-// (sdf/program.cpp:478 laneSourceOf): the leaf that decides the value, the
-// leaf across the first smooth band and its share.
-__device__ __forceinline__ void sourceOf(const GpuStep* __restrict__ code, const SsaOps* __restrict__ ssa, uint32_t count, uint32_t result, float* v, const float p[3], uint32_t& leaf, uint32_t& other, float& share) {
-	for (uint32_t i = 0; i < count; ++i) {
+// Every step's value by step number (unless v holds them), then the walk back
+// through the joins (sdf/program.cpp:478 laneSourceOf): the leaf that decides
+// the value, the leaf across the first smooth band and its share.
+__device__ __forceinline__ void sourceOf(bool held, const GpuStep* __restrict__ code, const SsaOps* __restrict__ ssa, uint32_t count, uint32_t result, float* v, const float p[3], uint32_t& leaf, uint32_t& other, float& share) {
+	for (uint32_t i = 0; i < (held ? 0u : count); ++i) {
 		const GpuStep s = code[i];
 		const SsaOps o  = ssa[i];
 		v[i]            = stepValue(s.op, v[o.a], v[o.b], v[o.c], s.value, p);
