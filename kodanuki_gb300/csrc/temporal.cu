@@ -84,12 +84,28 @@ __device__ __forceinline__ Plane planeThrough(const Surf& s, D eye, D heading, d
 
 __device__ __forceinline__ bool sameLeaf(uint32_t a, uint32_t b, bool recounted) { return recounted ? ((a == kSky) == (b == kSky)) : a == b; }
 
-// :397 onPlane
-__device__ __forceinline__ bool onPlane(const Plane& p, const Plane& other, bool recounted) {
-	if (!sameLeaf(other.leaf, p.leaf, recounted)) return false;
+// :397 onPlane, of a surface seen along a heading from an eye.  Both tests are
+// made in FP32 first, whose error here is below the bands left out (1e-6 of a
+// dot of unit normals, 2e-6 of the lengths a point is made of): what falls in
+// a band, or is not a number, is worked out in double.
+__device__ __forceinline__ bool onPlane(const Plane& p, const Surf& other, D eye, D heading, bool recounted) {
+	if (!sameLeaf(skyOf(other) ? kSky : other.leaf, p.leaf, recounted)) return false;
 	if (p.leaf == kSky) return true;
-	if (dotD(other.normal, p.normal) < kNormalCosine) return false;
-	return fabs(dotD(other.point - p.point, p.normal)) <= p.reach;
+	const V n = { float(p.normal.x), float(p.normal.y), float(p.normal.z) };
+	const float alike = float(other.normal.x) * n.x + float(other.normal.y) * n.y + float(other.normal.z) * n.z;
+	if (alike < float(kNormalCosine) - 1e-5f) return false;
+	const D from       = eye - p.point;
+	const V h          = { float(heading.x), float(heading.y), float(heading.z) }, f = { float(from.x), float(from.y), float(from.z) };
+	const float share  = other.distance / sqrtf(h.x * h.x + h.y * h.y + h.z * h.z);
+	const float off    = fabsf((f.x + h.x * share) * n.x + (f.y + h.y * share) * n.y + (f.z + h.z * share) * n.z);
+	const float band   = 1e-5f * (fabsf(f.x) + fabsf(f.y) + fabsf(f.z) + other.distance), reach = float(p.reach);
+	if (alike > float(kNormalCosine) + 1e-5f) {
+		if (off < reach - band) return true;
+		if (off > reach + band) return false;
+	}
+	const Plane o = planeThrough(other, eye, heading, 0.0);
+	if (dotD(o.normal, p.normal) < kNormalCosine) return false;
+	return fabs(dotD(o.point - p.point, p.normal)) <= p.reach;
 }
 
 __device__ __forceinline__ float divisorOf(float albedo) { return albedo < kAlbedoFloor ? 1.0f : albedo; }
@@ -111,7 +127,7 @@ __device__ __forceinline__ size_t clampedPixel(int x, int y, int w, int h) {
 __device__ __forceinline__ bool sampleOnPlane(const TemporalArgs& a, const Plane& p, size_t k) {
 	const int x = int(k % size_t(a.width)), y = int(k / size_t(a.width));
 	const Surf s = surfAt(a.io.first_distance, a.io.first_normal, a.io.first_leaf, k);
-	return onPlane(p, planeThrough(s, d3(a.now.eye), filmHeading(a.now, double(x) + double(a.centre[0]), double(y) + double(a.centre[1])), kDepthShare), false);
+	return onPlane(p, s, d3(a.now.eye), filmHeading(a.now, double(x) + double(a.centre[0]), double(y) + double(a.centre[1])), false);
 }
 
 __global__ void temporalKernel(TemporalArgs a) {
@@ -134,8 +150,11 @@ __global__ void temporalKernel(TemporalArgs a) {
 		const Surf first  = surfAt(io.first_distance, io.first_normal, io.first_leaf, k);
 		const Surf centre = surfAt(io.centre_distance, io.centre_normal, io.centre_leaf, k);
 		const bool aimed  = (skyOf(first) ? kSky : first.leaf) == (skyOf(centre) ? kSky : centre.leaf);
-		const D heading   = filmHeading(a.now, double(x) + double(a.centre[0]), double(y) + double(a.centre[1]));
-		const Plane plane = planeThrough(centre, d3(a.now.eye), heading, kDepthShare);
+		// the pixel's plane, where it is asked for: a camera that moved, a sample
+		// that missed the G-buffer's surface (the rate of double is a 64th of
+		// FP32's, and its root and quotient were most of a still frame's time)
+		const auto headingOf = [&] { return filmHeading(a.now, double(x) + double(a.centre[0]), double(y) + double(a.centre[1])); };
+		const auto planeOf   = [&](D heading) { return planeThrough(centre, d3(a.now.eye), heading, kDepthShare); };
 		// the history
 		bool found = false;
 		V history  = { 0, 0, 0 };
@@ -151,6 +170,8 @@ __global__ void temporalKernel(TemporalArgs a) {
 				}
 			} else {
 				// :584 surfacedHistory, :418 placeBefore, :495 fetchedHistory
+				const D heading    = headingOf();
+				const Plane plane  = planeOf(heading);
 				const D along      = plane.leaf == kSky ? heading : plane.point - d3(a.before.eye);
 				const double ahead = dotD(along, d3(a.before.forward));
 				if (ahead > 0) {
@@ -173,9 +194,8 @@ __global__ void temporalKernel(TemporalArgs a) {
 								const float lastLength = io.before_length[c];
 								if (!(lastLength > 0.0f)) continue;
 								const Surf last = surfAt(io.before_distance, io.before_normal, io.before_leaf, c);
-								const Plane lastPlane = planeThrough(last, d3(a.before.eye),
-								                                     filmHeading(a.before, double(cx) + double(a.centreBefore[0]), double(cy) + double(a.centreBefore[1])), 0.0);
-								if (!onPlane(plane, lastPlane, a.recounted != 0)) continue;
+								const D lastHeading = filmHeading(a.before, double(cx) + double(a.centreBefore[0]), double(cy) + double(a.centreBefore[1]));
+								if (!onPlane(plane, last, d3(a.before.eye), lastHeading, a.recounted != 0)) continue;
 								const float* lc = io.before_colour + 3 * c;
 								colour = colour + D { double(lc[0]), double(lc[1]), double(lc[2]) } * w;
 								moment += double(io.before_moment[c]) * w;
@@ -198,7 +218,13 @@ __global__ void temporalKernel(TemporalArgs a) {
 		float moment, length;
 		if (!found) {
 			// :796 freshBlend; not aimed: :754 jointFilled
-			if (aimed || sampleOnPlane(a, plane, size_t(k))) {
+			bool own = aimed;
+			Plane plane {};
+			if (!aimed) {
+				plane = planeOf(headingOf());
+				own   = sampleOnPlane(a, plane, size_t(k));
+			}
+			if (own) {
 				colour = sampleLight(io, size_t(k));
 			} else {
 				V fill = { 0, 0, 0 };
