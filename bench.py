@@ -51,8 +51,8 @@ DENOISE = True  # the temporal member and the a-trous denoiser on the frame's FP
 # smsp__inst_executed.sum, with the frame's own program-step counters): the
 # lane instructions the kernel issues a march-form program step, and the
 # warp execution efficiency (active lanes an instruction / 32).
-TRACE_LANE_INST_PER_PROGRAM_STEP = 156.9
-TRACE_WARP_EFFICIENCY = 0.249
+TRACE_LANE_INST_PER_PROGRAM_STEP = 79.0
+TRACE_WARP_EFFICIENCY = 0.401
 SM_COUNT, LANES_PER_SM = 152, 128
 BUILD = dict(min_depth=7, max_depth=11, split_steps=32)
 
@@ -240,7 +240,7 @@ def run_gpu(args) -> None:
     e_dt = time.perf_counter() - e0
     e2e = samples * world / e_dt / 1e6
 
-    # roofline of the dominant kernel, the sphere-trace kernel (90% of the
+    # roofline of the dominant kernel, the sphere-trace kernel (72% of the
     # frame's launch time): FP32 issue.  Its lane instructions a second are
     # the march-form program steps it ran in the timed frames, counted live,
     # times the lane instructions a step, over the frames' device time (its
@@ -283,7 +283,7 @@ def run_gpu(args) -> None:
             "algorithmic": f"{program / max(1, segments):.0f} march-form program steps a ray x {TRACE_LANE_INST_PER_PROGRAM_STEP} lane instructions a step (ncu); "
                            f"{rays_per_launch:.0f} rays a launch" if rays_per_launch else None,
             "note": "traffic: none against this roof (the kernel's DRAM bytes, from an ncu capture of one launch, are in the trace kernel's "
-                    "profile); the kernel issues at ~8 of 32 lanes (warp_efficiency), so its issue slots bind long before its FP32 lanes",
+                    "profile); the kernel issues at ~13 of 32 lanes (warp_efficiency), so its issue slots bind long before its FP32 lanes",
         }
         # over the frame's device time: the two render lanes' trace
         # launches overlap, so their summed launch time exceeds it

@@ -256,11 +256,12 @@ struct Pool {
 	uint32_t taken[32];      // the rays of this turn
 };
 
-// Four blocks an SM: 111 registers, 28 KB of shared memory and the slots'
-// columns a block.  Five leave less L1 (config 2's full frame 453 against 431 ms).
+// Four blocks an SM: 128 registers, 28 KB of shared memory and the slots'
+// columns a block.  Five leave less L1 (config 2's full frame 453 against 431
+// ms before a few rays were the whole warp's).
 // What bounds it: the issue of instructions while the SMs are full (51% of the
-// cycles, at 17 of 32 lanes), and in a launch by itself the last rays of it
-// (the SMs stand idle for 40% of 2.80 ms).
+// cycles, at 18 of 32 lanes), and in a launch by itself the last rays of it
+// (the SMs stand idle for 41% of 2.67 ms, 960 x 540 x 8 rays of config 2).
 __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_constant__ TraceArgs args) {
 	extern __shared__ float4 poolMemory[];
 	const DeviceWorld& w = args.world;
