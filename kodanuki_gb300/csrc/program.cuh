@@ -246,7 +246,9 @@ KDN_HD uint32_t unitsOf(const MarchStep& s) {
 }
 KDN_HD bool primitiveStep(const MarchStep& s) { return s.op < kMarchRare && (s.op & kMarchFormMask) == FormPrimitive; }
 
-// A primitive step at a point; last is the step before's result.
+// A primitive step at a point; last is the step before's result.  A post
+// operation's w that is a coordinate is the point's own: the column holds the
+// point only while a step that reads its slots runs.
 KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride, float px, float py, float pz, float last) {
 	const MarchParams c = paramsAt(unit);
 	MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
@@ -255,11 +257,19 @@ KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float
 	const uint32_t post = s.op & kMarchPostMask;
 	if (post != PostNone) {
 		float w = last;
-		if (!(s.m & PrimPrevious)) w = s.w == SlotImm ? s.value : slots[s.w * stride];
+		if (!(s.m & PrimPrevious)) w = s.w == SlotImm ? s.value : s.w == SlotX ? px : s.w == SlotY ? py : s.w == SlotZ ? pz : slots[s.w * stride];
 		r = posted(post, r, w, s.value, s.quarter);
 	}
 	if (s.m & PrimStored) slots[s.dst * stride] = r;
 	return r;
+}
+
+// A step as a turn of the march takes it: between turns a ray's column holds
+// the constants and what steps stored, but not the point.
+KDN_HD float programStep(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride, const float p[3], float last) {
+	if (primitiveStep(s)) return primitiveStepValue(s, unit, slots, stride, p[0], p[1], p[2], last);
+	setPoint(slots, stride, p);
+	return marchStep(s, unit, slots, stride);
 }
 
 // One program at one point; slots is its ray's column (stride the

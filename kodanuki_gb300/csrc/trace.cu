@@ -634,12 +634,7 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 				const MarchStep s     = w.march[pc];
 				const MarchStep* unit = w.march + pc + 1;
 				pc += unitsOf(s);
-				if (primitiveStep(s)) {
-					last = primitiveStepValue(s, unit, slots, kStride, p[0], p[1], p[2], last);
-				} else {
-					setPoint(slots, kStride, p);
-					last = marchStep(s, unit, slots, kStride);
-				}
+				last = programStep(s, unit, slots, kStride, p, last);
 				if (pc == end) {
 					programSteps += cost;
 					uint32_t k         = order >> 8 & 0xFFu;

@@ -1,9 +1,12 @@
 // kdn_world_march: the march form of a cell's kept programs, run on the host
-// by the same interpreter the trace kernel runs (program.cuh).
+// by the same interpreter the trace kernel runs (program.cuh), a step at a
+// time as its turns take them: what a step does not set itself or an earlier
+// one store is not in its ray's column (here it is not a number).
 #include "context.h"
 #include "locate.cuh"
 #include "program.cuh"
 
+#include <limits>
 #include <vector>
 
 using kdn::Context;
@@ -25,12 +28,20 @@ extern "C" kdn_status kdn_world_march(kdn_ctx* handle, uint64_t i, const float* 
 	const kdn::GpuLeaf& leaf = ctx->flat.leaves[size_t(~node)];
 	*programs                = leaf.count;
 	if (size_t(leaf.count) * n > capacity) return ctx->fail(KDN_BAD_ARG, "kdn_world_march: values too small");
-	std::vector<float> slots(kdn::kMaxSlots);
+	std::vector<float> slots(kdn::kMaxSlots, std::numeric_limits<float>::quiet_NaN());
 	kdn::setConstants(slots.data(), 1);
+	const float nowhere[3] = { slots[kdn::SlotX], slots[kdn::SlotX], slots[kdn::SlotX] };
 	for (uint32_t k = 0; k < leaf.count; ++k) {
 		const kdn::GpuProgram& g = ctx->flat.programs[leaf.first + k];
 		const kdn::MarchStep* code = ctx->flat.march.data() + g.march;
-		for (uint32_t j = 0; j < n; ++j) values[size_t(k) * n + j] = kdn::evalSlots(code, g.marchCount, slots.data(), 1, points + 3 * size_t(j));
+		for (uint32_t j = 0; j < n; ++j) {
+			float last = 0.0f;
+			for (uint32_t at = 0; at < g.marchCount; at += kdn::unitsOf(code[at])) {
+				kdn::setPoint(slots.data(), 1, nowhere);
+				last = kdn::programStep(code[at], code + at + 1, slots.data(), 1, points + 3 * size_t(j), last);
+			}
+			values[size_t(k) * n + j] = last;
+		}
 	}
 	return KDN_OK;
 }
