@@ -85,21 +85,26 @@ __device__ __forceinline__ Plane planeThrough(const Surf& s, D eye, D heading, d
 __device__ __forceinline__ bool sameLeaf(uint32_t a, uint32_t b, bool recounted) { return recounted ? ((a == kSky) == (b == kSky)) : a == b; }
 
 // :397 onPlane, of a surface seen along a heading from an eye.  Both tests are
-// made in FP32 first, whose error here is below the bands left out (1e-6 of a
-// dot of unit normals, 2e-6 of the lengths a point is made of): what falls in
-// a band, or is not a number, is worked out in double.
+// made in FP32 first, whose error here is below a tenth of the bands left out:
+// 1e-5 of the products a dot is made of, and of the lengths a point is made of
+// times the normal's (its largest part; a unit normal's bands are 1e-5 and 1e-5
+// of the lengths).  What falls in a band, is not a number, or is seen along a
+// heading whose square FP32 does not hold, is worked out in double.
 __device__ __forceinline__ bool onPlane(const Plane& p, const Surf& other, D eye, D heading, bool recounted) {
 	if (!sameLeaf(skyOf(other) ? kSky : other.leaf, p.leaf, recounted)) return false;
 	if (p.leaf == kSky) return true;
-	const V n = { float(p.normal.x), float(p.normal.y), float(p.normal.z) };
-	const float alike = float(other.normal.x) * n.x + float(other.normal.y) * n.y + float(other.normal.z) * n.z;
-	if (alike < float(kNormalCosine) - 1e-5f) return false;
+	const V n     = { float(p.normal.x), float(p.normal.y), float(p.normal.z) };
+	const V parts = { float(other.normal.x) * n.x, float(other.normal.y) * n.y, float(other.normal.z) * n.z };
+	const float alike = parts.x + parts.y + parts.z, loose = 1e-5f * fmaxf(1.0f, fabsf(parts.x) + fabsf(parts.y) + fabsf(parts.z));
+	if (alike < float(kNormalCosine) - loose) return false;
 	const D from       = eye - p.point;
 	const V h          = { float(heading.x), float(heading.y), float(heading.z) }, f = { float(from.x), float(from.y), float(from.z) };
-	const float share  = other.distance / sqrtf(h.x * h.x + h.y * h.y + h.z * h.z);
+	const float square = h.x * h.x + h.y * h.y + h.z * h.z;
+	const float share  = other.distance / sqrtf(square);
 	const float off    = fabsf((f.x + h.x * share) * n.x + (f.y + h.y * share) * n.y + (f.z + h.z * share) * n.z);
-	const float band   = 1e-5f * (fabsf(f.x) + fabsf(f.y) + fabsf(f.z) + other.distance), reach = float(p.reach);
-	if (alike > float(kNormalCosine) + 1e-5f) {
+	const float length = fmaxf(1.0f, fmaxf(fabsf(n.x), fmaxf(fabsf(n.y), fabsf(n.z))));
+	const float band   = 1e-5f * length * (fabsf(f.x) + fabsf(f.y) + fabsf(f.z) + fabsf(other.distance)), reach = float(p.reach);
+	if (alike > float(kNormalCosine) + loose && square > 1e-30f && square < 1e30f) {
 		if (off < reach - band) return true;
 		if (off > reach + band) return false;
 	}
