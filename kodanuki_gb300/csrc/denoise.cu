@@ -145,8 +145,13 @@ __global__ void __launch_bounds__(kBlockX * kBlockY) prepKernel(const __grid_con
 		const Pair scale  = lumaPair({ dv[0], 0.0f }, { dv[1], 0.0f }, { dv[2], 0.0f });
 		const Pair spread = add({ a.moment[p], 0.0f }, negative(mul(l, l)));
 		variance          = spread.h > 0.0f ? single(mul(spread, inverse(mul(mul(scale, scale), length)))) : 0.0f;
-		// a pair of an infinity is no number: plainly, then
-		if (!isfinite(variance) || !isfinite(a.moment[p])) variance = fmaxf(a.moment[p] - l.h * l.h, 0.0f) / (length * scale.h * scale.h);
+		// what a pair does not hold (an infinity, a square past FP32's range) is worked out in double
+		if (!isfinite(variance) || !isfinite(a.moment[p])) {
+			const double ld = 0.2126 * double(cr) + 0.7152 * double(cg) + 0.0722 * double(cb);
+			const double sd = 0.2126 * double(dv[0]) + 0.7152 * double(dv[1]) + 0.0722 * double(dv[2]);
+			const double apart = double(a.moment[p]) - ld * ld;
+			variance           = float((apart > 0.0 ? apart : 0.0) / (double(length) * sd * sd));
+		}
 	}
 	// a quotient of floats rounds as its double would, rounded
 	a.lightA[p] = make_float4(cr / dv[0], cg / dv[1], cb / dv[2], variance);
@@ -304,13 +309,16 @@ __global__ void __launch_bounds__(kBlockX * kBlockY) atrousKernel(const __grid_c
 		// remodulatedImage: share = 1 / (1 + length / 8)
 		const Pair share  = mul(inverse(sum(8.0f, a.length[p])), 8.0f);
 		const Pair rest   = add({ 1.0f, 0.0f }, negative(share));
-		const float plain = 8.0f / (8.0f + a.length[p]);
 		const float f[3]  = { l.x, l.y, l.z };
 		for (int ch = 0; ch < 3; ++ch) {
 			const float dv    = divisorOf(a.albedo[3 * p + ch]);
 			const Pair held   = a.demodulated ? product(a.colour[3 * p + ch], dv) : Pair { a.colour[3 * p + ch], 0.0f };
-			const float shown = single(add(mul(product(f[ch], dv), share), mul(held, rest)));
-			a.out[3 * p + ch] = isfinite(shown) ? shown : f[ch] * dv * plain + held.h * (1.0f - plain);
+			float shown       = single(add(mul(product(f[ch], dv), share), mul(held, rest)));
+			if (!isfinite(shown)) { // what a pair does not hold, in double
+				const double sd = 1.0 / (1.0 + double(a.length[p]) / 8.0), cd = double(a.colour[3 * p + ch]);
+				shown           = float(double(f[ch]) * double(dv) * sd + (a.demodulated ? cd * double(dv) : cd) * (1.0 - sd));
+			}
+			a.out[3 * p + ch] = shown;
 		}
 	}
 }
