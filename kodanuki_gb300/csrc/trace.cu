@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 	Pool& pool           = reinterpret_cast<Pool*>(poolMemory)[threadIdx.x / 32];
 	// a ray's register slots: a column each
 	float* const columns = reinterpret_cast<float*>(reinterpret_cast<Pool*>(poolMemory) + kWarps) + threadIdx.x / 32 * kPool;
-	// capped rays in the low 16 bits, carried ones in the high: one register
+	// a lane's capped rays in the low 16 bits, its carried ones in the high: one register
 	uint32_t marchSteps = 0, programSteps = 0, traced = 0, cappedCarried = 0, longest = 0;
 	// the steps a ray may take in this launch: a launch's budget, or the cap
 	const uint32_t allowance = args.budget > 0 ? args.budget : kMarchSteps;
@@ -769,21 +769,23 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 		__syncwarp();
 	}
 	if (args.counters) {
-		// one add per warp
+		// one add per warp (whose counts together are past 16 bits)
+		uint32_t capped = cappedCarried & 0xFFFFu, carried = cappedCarried >> 16;
 		for (int o = 16; o > 0; o >>= 1) {
 			marchSteps += __shfl_down_sync(0xFFFFFFFFu, marchSteps, o);
 			programSteps += __shfl_down_sync(0xFFFFFFFFu, programSteps, o);
 			traced += __shfl_down_sync(0xFFFFFFFFu, traced, o);
-			cappedCarried += __shfl_down_sync(0xFFFFFFFFu, cappedCarried, o);
+			capped += __shfl_down_sync(0xFFFFFFFFu, capped, o);
+			carried += __shfl_down_sync(0xFFFFFFFFu, carried, o);
 			longest = max(longest, __shfl_down_sync(0xFFFFFFFFu, longest, o));
 		}
 		if ((threadIdx.x & 31) == 0) {
 			atomicAdd(&args.counters[0], (unsigned long long) marchSteps);
 			atomicAdd(&args.counters[1], (unsigned long long) programSteps);
 			atomicMax(&args.counters[2], (unsigned long long) longest);
-			atomicAdd(&args.counters[3], (unsigned long long) (cappedCarried & 0xFFFFu));
+			atomicAdd(&args.counters[3], (unsigned long long) capped);
 			atomicAdd(&args.counters[4], (unsigned long long) traced);
-			if (cappedCarried >> 16) atomicAdd(&args.counters[5], (unsigned long long) (cappedCarried >> 16));
+			if (carried) atomicAdd(&args.counters[5], (unsigned long long) carried);
 		}
 	}
 }
