@@ -1378,13 +1378,16 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 			}
 			return o.slot;
 		};
+		// a coordinate a primitive is joined with: the plane through the origin
+		// before it (a primitive's turn does not put the point in its ray's column)
+		const bool joined = x.form == FormPrimitive && usesW && Fusing::point(x.w);
 		const bool sized = x.form == FormPrimitive && !(x.half[0] == 0.0f && x.half[1] == 0.0f && x.half[2] == 0.0f && x.round == 0.0f && std::signbit(x.round));
 		if (x.form == FormPrimitive) {
 			g.a     = x.terms[0];
 			g.b     = x.terms[1];
 			g.c     = x.terms[2];
 			g.flags = x.flags;
-			g.m     = uint8_t(x.kind | (sized ? PrimSized : 0) | (usesW && x.w.kind == Operand::Node && x.w.node == before ? PrimPrevious : 0) | (stored[j] ? PrimStored : 0));
+			g.m     = uint8_t(x.kind | (sized ? PrimSized : 0) | (joined || (usesW && x.w.kind == Operand::Node && x.w.node == before) ? PrimPrevious : 0) | (stored[j] ? PrimStored : 0));
 		} else {
 			g.a = slotOf(x.a);
 			if (x.form != FormRepeat) {
@@ -1416,8 +1419,6 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 		}
 		if (lastRead[j] == j) freeSlots.push_back(slot[j]);
 		g.dst = slot[j];
-		steps.push_back(g);
-		++kept;
 		const auto unit = [&](float v0, float v1, float v2, float v3) {
 			const float v[4] = { v0, v1, v2, v3 };
 			MarchStep u;
@@ -1426,6 +1427,17 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 			steps.push_back(u);
 			++kept;
 		};
+		if (joined) {
+			MarchStep plane = {};
+			plane.op        = FormPrimitive;
+			plane.a         = uint8_t(x.w.slot - SlotX);
+			plane.m         = PrimPlain;
+			steps.push_back(plane);
+			++kept;
+			unit(0.0f, 0.0f, 0.0f, 0.0f);
+		}
+		steps.push_back(g);
+		++kept;
 		if (x.form == FormPrimitive) unit(x.centre[0], x.centre[1], x.centre[2], x.params[3]);
 		if (sized) unit(x.half[0], x.half[1], x.half[2], x.round);
 		if (x.form == FormNorm) unit(x.params[0], 0.0f, 0.0f, 0.0f);

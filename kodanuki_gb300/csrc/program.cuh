@@ -247,8 +247,8 @@ KDN_HD uint32_t unitsOf(const MarchStep& s) {
 KDN_HD bool primitiveStep(const MarchStep& s) { return s.op < kMarchRare && (s.op & kMarchFormMask) == FormPrimitive; }
 
 // A primitive step at a point; last is the step before's result.  A post
-// operation's w that is a coordinate is the point's own: the column holds the
-// point only while a step that reads its slots runs.
+// operation's w is that, the immediate or a slot of the program's, never the
+// point's (the lowering makes a coordinate a plane of its own).
 KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float* slots, uint32_t stride, float px, float py, float pz, float last) {
 	const MarchParams c = paramsAt(unit);
 	MarchParams h { { 0.0f, 0.0f, 0.0f, -0.0f } };
@@ -257,7 +257,7 @@ KDN_HD float primitiveStepValue(const MarchStep& s, const MarchStep* unit, float
 	const uint32_t post = s.op & kMarchPostMask;
 	if (post != PostNone) {
 		float w = last;
-		if (!(s.m & PrimPrevious)) w = s.w == SlotImm ? s.value : s.w == SlotX ? px : s.w == SlotY ? py : s.w == SlotZ ? pz : slots[s.w * stride];
+		if (!(s.m & PrimPrevious)) w = s.w == SlotImm ? s.value : slots[s.w * stride];
 		r = posted(post, r, w, s.value, s.quarter);
 	}
 	if (s.m & PrimStored) slots[s.dst * stride] = r;

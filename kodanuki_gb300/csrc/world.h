@@ -41,7 +41,8 @@ enum Op : uint8_t {
 //    part, or the one slab itself; a box's inside term; and - e.  A plane, a
 //    sphere, and a rounded box with the faces, edges and corners a cut leaves
 //    of it are one step each, the same operations for all of them, so a warp
-//    whose lanes are at different ones does not split;
+//    whose lanes are at different ones does not split; a coordinate one is
+//    joined with is a plane of its own before it;
 //  - FormNorm: such a root over slots, where other steps read the slabs too
 //    or make them;
 //  - FormRepeat: a coordinate taken into the middle cell of a repetition,
