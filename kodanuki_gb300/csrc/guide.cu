@@ -98,13 +98,15 @@ __device__ __forceinline__ uint64_t descOf(uint32_t addr, uint32_t K) {
 // instruction descriptor of kind::f16: FP32 D, BF16 A and B, both K-major, M 128
 __device__ __forceinline__ uint32_t idescOf(uint32_t N) { return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24); }
 
-// D[128 x N] = A[128 x K] . B[N x K]^T, 16 of K an instruction
-__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t K, uint32_t N) {
+// D[128 x N] = A[128 x K] . B[N x K]^T, 16 of K an instruction; onto what D
+// holds where it is not the first
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t K, uint32_t N, bool first = true) {
 	const uint32_t idesc = idescOf(N);
 	for (uint32_t kk = 0; kk < K / 16u; ++kk) {
 		const uint64_t ad = descOf(a + kk * 256u, K);
 		const uint64_t bd = descOf(b + kk * 256u, K);
-		asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(kk) : "memory");
+		const uint32_t on = first ? kk : 1u;
+		asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(on) : "memory");
 	}
 }
 __device__ __forceinline__ void commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
@@ -147,43 +149,40 @@ __device__ __forceinline__ void tload(uint32_t tmem, uint32_t col, float* v) {
 	for (int c = 0; c < N; c += 16) tload16(tmem + (lane << 16) + col + c, v + c);
 }
 
-template <int K>
-__device__ __forceinline__ void storeRow(uint8_t* img, uint32_t r, const float* v, bool relu) {
+// N columns from k0 on of row r of an image of K columns, and of column c of a
+// transposed image
+template <int K, int N>
+__device__ __forceinline__ void storeRow(uint8_t* img, uint32_t r, uint32_t k0, const float* v, bool relu) {
 #pragma unroll
-	for (int k0 = 0; k0 < K; k0 += 8) {
+	for (int k = 0; k < N; k += 8) {
 		uint32_t p[4];
 #pragma unroll
 		for (int j = 0; j < 4; ++j) {
-			float a = v[k0 + 2 * j], b = v[k0 + 2 * j + 1];
-			if (relu) {
-				a = fmaxf(a, 0.0f);
-				b = fmaxf(b, 0.0f);
-			}
-			__nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+			const float x = relu ? fmaxf(v[k + 2 * j], 0.0f) : v[k + 2 * j], y = relu ? fmaxf(v[k + 2 * j + 1], 0.0f) : v[k + 2 * j + 1];
+			__nv_bfloat162 h = __floats2bfloat162_rn(x, y);
 			p[j]             = *reinterpret_cast<uint32_t*>(&h);
 		}
-		*reinterpret_cast<uint4*>(img + imgAt(r, k0, K)) = make_uint4(p[0], p[1], p[2], p[3]);
+		*reinterpret_cast<uint4*>(img + imgAt(r, k0 + k, K)) = make_uint4(p[0], p[1], p[2], p[3]);
 	}
 }
-template <int K>
-__device__ __forceinline__ void readRow(const uint8_t* img, uint32_t r, float* v) {
+template <int N>
+__device__ __forceinline__ void storeColumn(uint8_t* img, uint32_t c, uint32_t f0, const float* v) {
 #pragma unroll
-	for (int k0 = 0; k0 < K; k0 += 8) {
-		const uint4 q      = *reinterpret_cast<const uint4*>(img + imgAt(r, k0, K));
+	for (int f = 0; f < N; ++f) *reinterpret_cast<__nv_bfloat16*>(img + imgAt(f0 + f, c, 128)) = __float2bfloat16_rn(v[f]);
+}
+template <int K, int N>
+__device__ __forceinline__ void readRow(const uint8_t* img, uint32_t r, uint32_t k0, float* v) {
+#pragma unroll
+	for (int k = 0; k < N; k += 8) {
+		const uint4 q       = *reinterpret_cast<const uint4*>(img + imgAt(r, k0 + k, K));
 		const uint32_t p[4] = { q.x, q.y, q.z, q.w };
 #pragma unroll
 		for (int j = 0; j < 4; ++j) {
 			__nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&p[j]);
-			v[k0 + 2 * j]     = __bfloat162float(h.x);
-			v[k0 + 2 * j + 1] = __bfloat162float(h.y);
+			v[k + 2 * j]     = __bfloat162float(h.x);
+			v[k + 2 * j + 1] = __bfloat162float(h.y);
 		}
 	}
-}
-// column c of a transposed image [F][128]: row f gets v[f]
-template <int F>
-__device__ __forceinline__ void storeColumn(uint8_t* img, uint32_t c, const float* v) {
-#pragma unroll
-	for (int f = 0; f < F; ++f) *reinterpret_cast<__nv_bfloat16*>(img + imgAt(f, c, 128)) = __float2bfloat16_rn(v[f]);
 }
 
 struct Region {
@@ -369,53 +368,6 @@ constexpr uint32_t kTmemDX = 128, kTmemDW = 192;
 // One 16-column slice of this thread's TMEM lane.
 __device__ __forceinline__ void tslice(uint32_t tmem, uint32_t col, float* v) { tload16(tmem + (((threadIdx.x >> 5) & 3u) * 32u << 16) + col, v); }
 
-// N columns from k0 on of row r of an image of K columns, and of column c of a
-// transposed image
-template <int K, int N>
-__device__ __forceinline__ void storePart(uint8_t* img, uint32_t r, uint32_t k0, const float* v, bool relu) {
-#pragma unroll
-	for (int k = 0; k < N; k += 8) {
-		uint32_t p[4];
-#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			const float x = relu ? fmaxf(v[k + 2 * j], 0.0f) : v[k + 2 * j], y = relu ? fmaxf(v[k + 2 * j + 1], 0.0f) : v[k + 2 * j + 1];
-			__nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-			p[j]             = *reinterpret_cast<uint32_t*>(&h);
-		}
-		*reinterpret_cast<uint4*>(img + imgAt(r, k0 + k, K)) = make_uint4(p[0], p[1], p[2], p[3]);
-	}
-}
-template <int N>
-__device__ __forceinline__ void storeColumnPart(uint8_t* img, uint32_t c, uint32_t f0, const float* v) {
-#pragma unroll
-	for (int f = 0; f < N; ++f) *reinterpret_cast<__nv_bfloat16*>(img + imgAt(f0 + f, c, 128)) = __float2bfloat16_rn(v[f]);
-}
-template <int K, int N>
-__device__ __forceinline__ void readPart(const uint8_t* img, uint32_t r, uint32_t k0, float* v) {
-#pragma unroll
-	for (int k = 0; k < N; k += 8) {
-		const uint4 q       = *reinterpret_cast<const uint4*>(img + imgAt(r, k0 + k, K));
-		const uint32_t p[4] = { q.x, q.y, q.z, q.w };
-#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			__nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&p[j]);
-			v[k + 2 * j]     = __bfloat162float(h.x);
-			v[k + 2 * j + 1] = __bfloat162float(h.y);
-		}
-	}
-}
-
-// D += A . B^T over several instructions; first: the accumulator starts afresh
-__device__ __forceinline__ void mmaOnto(uint32_t d, uint32_t a, uint32_t b, uint32_t K, uint32_t N, bool first) {
-	const uint32_t idesc = idescOf(N);
-	for (uint32_t kk = 0; kk < K / 16u; ++kk) {
-		const uint64_t ad = descOf(a + kk * 256u, K);
-		const uint64_t bd = descOf(b + kk * 256u, K);
-		const uint32_t on = first ? kk : 1u;
-		asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(on) : "memory");
-	}
-}
-
 // A training step's gradients: a persistent CTA an SM takes tiles of 128
 // samples.  What bounds it is the table: 128 gathers and as many reductions of
 // two floats a sample, served by the L2; the rest is a chain of nine small
@@ -473,12 +425,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_con
 			v[2 * k]     = a;
 			v[2 * k + 1] = b;
 		}
-		storePart<48, 8>(X[0], row, group * 8u, v, false);
+		storeRow<48, 8>(X[0], row, group * 8u, v, false);
 		if (group == 3) {
 #pragma unroll
 			for (int k = 0; k < 16; ++k) v[k] = 0.0f;
 			if (live) v[0] = sample[3], v[1] = sample[4], v[2] = sample[5], v[3] = 1.0f;
-			storePart<48, 16>(X[0], row, 32u, v, false);
+			storeRow<48, 16>(X[0], row, 32u, v, false);
 		}
 		bool ok = loaded || waitBar(barLoad, 0);
 		loaded  = true;
@@ -498,7 +450,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_con
 			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 			if (l < 3) {
 				tslice(tmem, 64u * (l & 1) + group * 16u, v);
-				storePart<64, 16>(X[l + 1], row, group * 16u, v, true);
+				storeRow<64, 16>(X[l + 1], row, group * 16u, v, true);
 				stage();
 			}
 		}
@@ -513,8 +465,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_con
 #pragma unroll
 					for (int k = 0; k < 48; ++k) g[k] = 0.0f;
 				}
-				storeRow<48>(DY, row, g, false);
-				storeColumn<48>(DYT, row, g);
+				storeRow<48, 48>(DY, row, 0, g, false);
+				storeColumn<48>(DYT, row, 0, g);
 				lossSum += rowLoss;
 			}
 			stage();
@@ -526,14 +478,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_con
 			const uint32_t k0 = group * 16u;
 			float xr[16];
 			if (k0 < nIn(l)) {
-				if (l == 0) readPart<48, 16>(X[0], row, k0, xr);
-				else readPart<64, 16>(X[l], row, k0, xr);
-				storeColumnPart<16>(XT, row, k0, xr);
+				if (l == 0) readRow<48, 16>(X[0], row, k0, xr);
+				else readRow<64, 16>(X[l], row, k0, xr);
+				storeColumn<16>(XT, row, k0, xr);
 			}
 			stage();
 			if (tid == 0) {
 				mma(tmem + kTmemDX, sAddr(DY), sAddr(sm + imgWt(l)), nOut(l), nIn(l));
-				mmaOnto(tmem + kTmemDW + 64u * l, sAddr(DYT), sAddr(XT), 128u, nIn(l), first);
+				mma(tmem + kTmemDW + 64u * l, sAddr(DYT), sAddr(XT), 128u, nIn(l), first);
 				commit(barMma);
 			}
 			ok = waitBar(barMma, phase);
@@ -544,8 +496,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) trainKernel(const __grid_con
 				tslice(tmem, kTmemDX + k0, v);
 #pragma unroll
 				for (int k = 0; k < 16; ++k) v[k] = xr[k] > 0.0f ? v[k] : 0.0f;
-				storePart<64, 16>(DY, row, k0, v, false);
-				storeColumnPart<16>(DYT, row, k0, v);
+				storeRow<64, 16>(DY, row, k0, v, false);
+				storeColumn<16>(DYT, row, k0, v);
 			} else {
 				tslice(tmem, kTmemDX + (group >> 1) * 16u, v);
 				if (live) {
@@ -650,7 +602,7 @@ __global__ void __launch_bounds__(128) queryKernel(const __grid_constant__ Query
 #pragma unroll
 			for (int k = 0; k < int(kIn); ++k) v[k] = 0.0f;
 		}
-		storeRow<48>(X0, tid, v, false);
+		storeRow<48, 48>(X0, tid, 0, v, false);
 		if (!loaded) {
 			loaded = true;
 			failed = __syncthreads_or(!waitBar(barLoad, 0));
@@ -671,7 +623,7 @@ __global__ void __launch_bounds__(128) queryKernel(const __grid_constant__ Query
 			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 			if (l < 3) {
 				tload<64>(tmem, 64u * (l & 1), v);
-				storeRow<64>(out[l], tid, v, true);
+				storeRow<64, 64>(out[l], tid, 0, v, true);
 			} else {
 				tload<48>(tmem, 64u, v);
 			}

@@ -557,14 +557,13 @@ struct Node {
 	bool negation = false; // fma(x, -1, 0): -x
 	bool product  = false; // fma(x, y, 0) from a multiplication
 	// a fused step (world.h MarchForm): its parameters as they are written,
-	// how far an axis has come (the terms taken so far), and the single steps
-	// it stands for
+	// how far an axis has come (the terms taken so far)
 	uint8_t form  = FormFma, flags = 0;
 	bool inside = false;   // FormNorm: an inside term, m
 	Operand m;
 	float params[4] = { 0.0f, 0.0f, -0.0f, 0.0f };
 	uint8_t stage = 0;     // FormAxis: 0 none, 1 c, 2 a side, 3 h, 4 r, 5 e; else 1 once e is taken
-	uint32_t took = 1;
+	bool more = false;     // a slab that stands for more than one single step
 	// FormPrimitive: its flags, its terms (axis and side), their c, h and r (params[3] is e)
 	uint8_t kind = 0, terms[3] = { 0, 0, 0 };
 	float centre[3] = { 0.0f, 0.0f, 0.0f }, half[3] = { 0.0f, 0.0f, 0.0f }, round = -0.0f;
@@ -729,14 +728,11 @@ struct Fusing {
 			if (!copyOf(*s[k], q[k]) || !readsW(*s[k]) || s[k]->w.kind != Operand::Immediate || s[k]->w.value != 0.0) return;
 		}
 		if (!((s[0]->post == PostMax && s[1]->post == PostMin) || (s[0]->post == PostMin && s[1]->post == PostMax)) || !same(q[0], q[1])) return;
-		const uint32_t took = n.took + s[0]->took + s[1]->took;
 		if (const Node* whole = only(q[0], 2); whole && n.post == PostNone) {
 			n = *whole;
-			n.took += took;
 		} else {
-			n.a    = q[0];
-			n.c    = Operand();
-			n.took = took;
+			n.a = q[0];
+			n.c = Operand();
 		}
 	}
 
@@ -780,7 +776,7 @@ struct Fusing {
 		for (int k = 0; k < 4; ++k) f.params[k] = before->params[k];
 		f.a     = before->a;
 		f.flags = before->flags;
-		f.took  = before->took + n.took;
+		f.more  = true;
 		if (negated || copied) {
 			if (stage != 1 || (copied && n.post != PostAbs)) return;
 			f.flags = negated ? SideNegative : SideAbs;
@@ -822,7 +818,6 @@ struct Fusing {
 		f.a      = n.c;
 		f.radius = scaled->a.value;
 		f.params[0] = float(offset);
-		f.took += scaled->took + whole->took + moved->took + over->took;
 		n = f;
 	}
 
@@ -832,7 +827,6 @@ struct Fusing {
 		Operand x;
 		bool positive = false, fused = false;
 		Node* strip   = nullptr; // a step that loses its square
-		uint32_t took = 0;
 	};
 	bool term(const Operand& o, Term& t) const {
 		Node* n = only(o);
@@ -842,14 +836,11 @@ struct Fusing {
 			if (!copyOf(*n, t.x)) {
 				t.x     = o;
 				t.strip = n;
-			} else {
-				t.took = n->took;
 			}
 			return true;
 		}
 		if (n->post == PostNone && n->form == FormFma && same(n->a, n->b) && n->a.kind == Operand::Node && is(n->c, SlotZero)) {
-			t.x    = n->a;
-			t.took = n->took;
+			t.x = n->a;
 			return true;
 		}
 		return false;
@@ -884,10 +875,7 @@ struct Fusing {
 		}
 		const Node* s = only(rest);
 		if (!s || s->post != PostNone || out.size() > 2) return false;
-		const size_t at = out.size();
-		if (!terms(*s, out)) return false;
-		out[at].took += s->took;
-		return true;
+		return terms(*s, out);
 	}
 	void norm(Node& n) {
 		std::vector<Term> t;
@@ -905,7 +893,6 @@ struct Fusing {
 			f.flags |= uint8_t(SumHas0 << k);
 			if (t[k].positive) f.flags |= uint8_t(SumPositive0 << k);
 			if (t[k].fused) f.flags |= uint8_t(k == 1 ? SumFused1 : SumFused2);
-			f.took += t[k].took;
 		}
 		for (const Term& k : t) {
 			if (k.strip) k.strip->post = PostNone;
@@ -926,7 +913,7 @@ struct Fusing {
 			f.w      = n.w;
 			f.radius = n.radius;
 			f.stage  = 1;
-			f.took += n.took;
+			f.more  = true;
 			f.params[b->form == FormNorm ? 0 : 3] = float(value);
 			n = f;
 			return;
@@ -943,7 +930,6 @@ struct Fusing {
 			f.radius = n.radius;
 			f.inside = true;
 			f.m      = h;
-			f.took += n.took + m->took;
 			n = f;
 			return;
 		}
@@ -1000,7 +986,6 @@ struct Fusing {
 			f.centre[k] = x.params[0];
 			f.half[k]   = x.params[1];
 			f.terms[k]  = uint8_t(x.a.slot - SlotX) | uint8_t(x.flags << kTermSideShift);
-			f.took += x.took;
 		}
 		return true;
 	}
@@ -1064,7 +1049,6 @@ struct Fusing {
 			f.kind  = uint8_t(PrimSingle | PrimInside | (slabs == 3 ? PrimThird : 0));
 			f.stage = 0;
 			f.params[3] = 0.0f;
-			f.took += most->took + least->took;
 			if (termed(f, s)) {
 				n = f;
 				return;
@@ -1087,7 +1071,7 @@ struct Fusing {
 		f.post   = n.post;
 		f.w      = w;
 		f.radius = n.radius;
-		f.took += n.took;
+		f.more   = true;
 		n = f;
 	}
 
@@ -1131,7 +1115,7 @@ struct Fusing {
 		}
 		for (size_t j = 0; j < nodes.size(); ++j) {
 			Node& n = nodes[j];
-			if (!taken[j] || n.form != FormPrimitive || n.kind != PrimPlain || n.took != 1) continue;
+			if (!taken[j] || n.form != FormPrimitive || n.kind != PrimPlain || n.more) continue;
 			const Operand x = reserved(uint8_t(SlotX + (n.terms[0] & 3))), c = immediate(n.centre[0]);
 			const uint8_t side = n.terms[0] >> kTermSideShift;
 			n.form             = FormFma;
@@ -1546,16 +1530,13 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 		for (size_t k = 0; k < c.programs.size(); ++k) flat.programs.push_back(programs[named[at++]]);
 		leaf.shape     = ShapePrograms;
 		if (c.occupancy == Empty || leaf.count == 0) {
-			leaf.shape     = ShapeEmpty;
-			leaf.params[0] = -std::numeric_limits<float>::infinity();
-			leaf.params[2] = -0.0f;
+			leaf.shape = ShapeEmpty;
 		} else {
 			const GpuProgram& g = flat.programs[leaf.first];
 			leaf.march          = g.march;
 			leaf.marchCount     = g.marchCount;
 			leaf.marchSteps     = g.marchSteps;
 			const MarchStep& s  = flat.march[g.march];
-			std::memcpy(leaf.params, &s, sizeof leaf.params);
 			if (leaf.count == 1 && s.op == FormPrimitive && g.marchCount == (s.m & PrimSized ? 3 : 2)) {
 				float c[4], h[4] = { 0.0f, 0.0f, 0.0f, -0.0f };
 				std::memcpy(c, &flat.march[g.march + 1], sizeof c);

@@ -38,7 +38,7 @@ struct BuildOptions {
 	int min_depth        = 6;
 	int max_depth        = 10;
 	uint32_t split_steps = 96;
-	size_t max_cells     = size_t(1) << 26;
+	size_t max_cells     = size_t(kMostCells);
 };
 
 struct FlatWorld {

@@ -48,7 +48,8 @@ enum Op : uint8_t {
 //  - FormRepeat: a coordinate taken into the middle cell of a repetition,
 //    x - s * floor(x / s + o).
 // 98% of the programs the march runs on config 2 and the city are primitives
-// alone, joined by the post operations.
+// alone, joined by the post operations.  A slab that is one single step and is
+// read by other forms stays that step.
 enum MarchPost : uint8_t { PostNone, PostSqrt, PostAbs, PostPosSq, PostMin, PostMax, PostSminK };
 enum MarchForm : uint8_t { FormFma = 0, FormAxis = 8, FormPrimitive = 16, FormNorm = 24, FormRepeat = 32 }; // op = form + post; FormAxis: in the lowering alone
 constexpr uint8_t kMarchPostMask = 7, kMarchFormMask = 56;
@@ -117,7 +118,7 @@ struct alignas(16) GpuProgram {
 	uint16_t result;     // SSA index of the result
 	uint8_t slot;        // slot of the result
 	uint8_t slots;       // slots used
-	uint16_t marchCount; // units of the march form (a fused step takes two)
+	uint16_t marchCount; // units of the march form (a fused step takes two or three)
 	uint32_t object;     // index into the scene's object programs
 	uint32_t march;      // first MarchStep of the march form
 	uint16_t marchSlots; // slots the march form uses
@@ -130,8 +131,7 @@ enum Occupancy : uint8_t { Empty = 0, Filled = 1, Surface = 2 };
 
 // A leaf.  An empty one, or one whose one program is a single axis or sphere
 // (on config 2, 54% and 34% of the march's steps; on a ray that skims the
-// ground, all of them), is marched from the record itself, in registers: an
-// empty leaf is an axis infinitely far from its slab.
+// ground, all of them), is marched from the record itself, in registers.
 enum LeafShape : uint8_t { ShapeAxis = 0, ShapeSphere = 1, ShapePrograms = 2, ShapeEmpty = 3 }; // bits 0-1
 constexpr uint8_t kShapeMask = 3, kShapeAxisShift = 2, kShapeSideShift = 4; // an axis: bits 2-3 which, 4-5 its AxisSide
 struct alignas(16) GpuLeaf {
@@ -144,9 +144,7 @@ struct alignas(16) GpuLeaf {
 	uint32_t march;
 	uint16_t marchCount;
 	uint16_t marchSteps;
-	// of an axis c, h, r, e; of a sphere its centre and radius; of programs the
-	// first one's first unit (MarchStep)
-	float params[4];
+	float params[4]; // of an axis c, h, r, e; of a sphere its centre and radius
 };
 static_assert(sizeof(GpuLeaf) == 32, "GpuLeaf is 32 bytes");
 
@@ -169,6 +167,7 @@ static_assert(sizeof(GpuLeaf) == 32, "GpuLeaf is 32 bytes");
 constexpr uint32_t kEntryLeaf = 1u << 31, kEntryEmpty = 1u << 30, kEntryLevelShift = 26, kEntryIndex = (1u << 26) - 1u;
 constexpr uint32_t kBrick = 64; // entries a brick, x fastest
 constexpr uint32_t kGridLevel = 7, kMostFine = 12;
+constexpr uint64_t kMostCells = uint64_t(kEntryIndex) + 1u; // cells a tree may have: an entry names any leaf
 
 // Everything the trace kernel reads, as device pointers.
 struct DeviceWorld {
