@@ -381,9 +381,10 @@ struct Pending {
 	Iv box[3];
 };
 
+// body(i, scratch) for i below n, `grain` of them at a time a thread.
 template <typename F>
-void parallelFor(size_t n, int threads, const F& body) {
-	if (threads <= 1 || n < 64) {
+void parallelFor(size_t n, int threads, const F& body, size_t grain = 16) {
+	if (threads <= 1 || n < 4 * grain) {
 		Scratch w;
 		for (size_t i = 0; i < n; ++i) body(i, w);
 		return;
@@ -394,9 +395,9 @@ void parallelFor(size_t n, int threads, const F& body) {
 		pool.emplace_back([&]() {
 			Scratch w;
 			for (;;) {
-				const size_t i = next.fetch_add(16);
+				const size_t i = next.fetch_add(grain);
 				if (i >= n) break;
-				for (size_t k = i; k < std::min(n, i + 16); ++k) body(k, w);
+				for (size_t k = i; k < std::min(n, i + grain); ++k) body(k, w);
 			}
 		});
 	}
@@ -1140,6 +1141,7 @@ std::string marchCode(const Prog& p, std::vector<MarchStep>& steps, GpuProgram& 
 	using namespace march;
 	const uint32_t n = uint32_t(p.steps.size());
 	Lowering L;
+	L.nodes.reserve(n + 8);
 	L.refUses.assign(n, 0);
 	for (uint32_t i = 0; i < n; ++i) {
 		const kdn_step& s    = p.steps[i];
@@ -1455,7 +1457,9 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 	}
 	// Compile them on every core: contiguous runs of the order, each into
 	// its own buffers (offsets from the run's start), then laid end to end
-	// in order, so the layout is the one a single thread would make.
+	// in order, so the layout is the one a single thread would make.  A run is
+	// a few milliseconds' work and is taken by itself (sixteen at a time left
+	// half of 16 cores without any, and small worlds to one of them).
 	struct Run {
 		size_t first, end;
 		std::vector<GpuProgram> programs;
@@ -1472,7 +1476,7 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 		runs[r].first = order.size() * r / runCount;
 		runs[r].end   = order.size() * (r + 1) / runCount;
 	}
-	parallelFor(runCount, runCount < 64 ? 1 : threads, [&](size_t r, Scratch&) {
+	parallelFor(runCount, threads, [&](size_t r, Scratch&) {
 		Run& run = runs[r];
 		run.programs.reserve(run.end - run.first);
 		for (size_t k = run.first; k < run.end; ++k) {
@@ -1486,7 +1490,7 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 			}
 			run.programs.push_back(g);
 		}
-	});
+	}, 1);
 	for (const Run& run : runs) {
 		if (!run.error.empty()) return run.error;
 	}
@@ -1502,7 +1506,7 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 	flat.steps.resize(stepTotal);
 	flat.ssa.resize(stepTotal);
 	flat.march.resize(marchTotal);
-	parallelFor(runCount, runCount < 64 ? 1 : threads, [&](size_t r, Scratch&) {
+	parallelFor(runCount, threads, [&](size_t r, Scratch&) {
 		const Run& run = runs[r];
 		std::copy(run.steps.begin(), run.steps.end(), flat.steps.begin() + std::ptrdiff_t(stepBase[r]));
 		std::copy(run.ssa.begin(), run.ssa.end(), flat.ssa.begin() + std::ptrdiff_t(stepBase[r]));
@@ -1513,7 +1517,7 @@ std::string flattenOctree(const Octree& tree, FlatWorld& flat) {
 			g.march += uint32_t(marchBase[r]);
 			programs[run.first + k] = g;
 		}
-	});
+	}, 1);
 	// the leaves; each names its programs through an indirection, and the
 	// kernel reads them as one run, so the GpuPrograms are laid out per leaf
 	flat.programs.reserve(named.size());
