@@ -51,8 +51,8 @@ DENOISE = True  # the temporal member and the a-trous denoiser on the frame's FP
 # smsp__inst_executed.sum, with the frame's own program-step counters): the
 # lane instructions the kernel issues a march-form program step, and the
 # warp execution efficiency (active lanes an instruction / 32).
-TRACE_LANE_INST_PER_PROGRAM_STEP = 79.0
-TRACE_WARP_EFFICIENCY = 0.401
+TRACE_LANE_INST_PER_PROGRAM_STEP = 78.2
+TRACE_WARP_EFFICIENCY = 0.397
 SM_COUNT, LANES_PER_SM = 152, 128
 BUILD = dict(min_depth=7, max_depth=11, split_steps=32)
 

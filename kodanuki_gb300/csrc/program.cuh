@@ -341,7 +341,8 @@ __device__ __forceinline__ DualF dualStep(uint8_t op, DualF a, DualF b, DualF c,
 
 // A step of the operations that distances are made of, worked out together and
 // the step's picked, so the lanes of a warp at different steps do not split;
-// dualStep's to the bit.  A gradient is fa * x.g, and + fb * b.g for a sum or a
+// dualStep's to the bit but for a product's gradient, whose two terms may be
+// fused the other way.  A gradient is fa * x.g, and + fb * b.g for a sum or a
 // product, x being an operand or a coordinate's own.
 __device__ __forceinline__ DualF commonDual(uint8_t op, DualF a, DualF b, float value, const float p[3]) {
 	const bool lesser = a.v <= b.v, greater = a.v >= b.v, negative = a.v < 0.0f;

@@ -38,7 +38,8 @@ constexpr uint64_t kPixelBytes = 128 + 116;
 // to the device's range by kdn_open_sharing).
 constexpr int kInteractivePriority = -8;
 // March steps a ray takes in one trace launch (kdn_set_march_budget) of an
-// interactive and of a batch request's frames
+// interactive and of a batch request's frames (set when a lone step took 1.8
+// us; it is 35 to 300 ns now, and the budgets are yet to be swept again)
 constexpr uint32_t kInteractiveMarchBudget = 64;
 constexpr uint32_t kBatchMarchBudget       = 1024;
 

@@ -793,9 +793,8 @@ __global__ void __launch_bounds__(kTraceBlock, 4) traceKernel(const __grid_const
 // A hit's normal and leaves: one walk over the winning program in duals, which
 // keeps every step's value for the walk back to the leaf.  What bounds it is
 // that a warp's hits are on different programs: the common operations are one
-// stretch of code for all (a million rays of config 2 and their hits 3.1
-// against 3.0 ms, the full frame 400 against 381 ms, the city 78 against 72.6
-// with a walk for the duals, one for the values and a switch).
+// stretch of code for all (config 2's full frame 400 against 381 ms, the city 78
+// against 72.6, with a walk for the duals, one for the values and a switch).
 __global__ void __launch_bounds__(kTraceBlock) hitKernel(HitArgs args) {
 	const DeviceWorld& w = args.world;
 	const uint32_t n     = args.count ? *args.count : args.n;
